@@ -1,0 +1,34 @@
+"""The native host path (csrc/torch_host.cpp): one C++ call per op for plain CUDA tensors, with or without autograd and under
+one ``torch.func.jvp``.  Its functions return None for everything else, and the caller takes the general route.
+
+With DMF_ATTN_CHECK=1 (which reads the device status word back after every call) every function returns None.
+"""
+
+from __future__ import annotations
+
+import importlib.util
+import os
+
+from . import _lib
+from . import build as _build
+
+
+def _load():
+    _lib.load()                    # libdmf_attn.so first: built if stale, ABI version checked
+    spec = importlib.util.spec_from_file_location("_dmf_torch", _build.build_host())
+    module = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(module)
+    return module
+
+
+_module = _load()
+launch_count, set_launch_count, set_status_word = _module.launch_count, _module.set_launch_count, _module.set_status_word
+
+# DMF_ATTN_CHECK=1 reads the status word back after every call (synchronises; for tests and debugging).
+CHECK_EVERY_CALL = os.environ.get("DMF_ATTN_CHECK", "0") == "1"
+
+if CHECK_EVERY_CALL:
+    attn_func = attn_qkvpacked = rms_norm = ln_modulate = gate_residual = lambda *args: None
+else:
+    attn_func, attn_qkvpacked = _module.attn_func, _module.attn_qkvpacked
+    rms_norm, ln_modulate, gate_residual = _module.rms_norm, _module.ln_modulate, _module.gate_residual

@@ -30,7 +30,7 @@ from typing import Optional
 import torch
 import torch.autograd.forward_ad as fwAD
 
-from . import _lib
+from . import _lib, _native
 from . import ops as _ops
 
 WIDTHS = (384, 768, 1024, 1152)   # hidden sizes the row kernels are compiled for (DMFT-S/B/L/XL)
@@ -261,6 +261,10 @@ def ln_modulate(x: torch.Tensor, shift: torch.Tensor, scale: torch.Tensor, eps: 
     """``F.layer_norm(x, (C,), eps=eps) * (1 + scale) + shift`` for x (B, L, C) and shift / scale (B, C) or
     (B, 1, C); dual tensors in give a dual tensor out.  The result has ``out_dtype`` (default: the autocast
     dtype when autocast is on, else x's dtype)."""
+    if not torch.compiler.is_compiling():
+        out = _native.ln_modulate(x, shift, scale, eps, out_dtype)
+        if out is not None:
+            return out
     if out_dtype is None:
         out_dtype = torch.get_autocast_dtype("cuda") if torch.is_autocast_enabled("cuda") else x.dtype
     xp, xt = fwAD.unpack_dual(x)
@@ -277,6 +281,10 @@ def ln_modulate(x: torch.Tensor, shift: torch.Tensor, scale: torch.Tensor, eps: 
 def gate_residual(x: torch.Tensor, gate: torch.Tensor, h: torch.Tensor) -> torch.Tensor:
     """``x + gate * h`` for x, h (B, L, C) and gate (B, C) or (B, 1, C); the result has x's dtype; dual tensors
     in give a dual tensor out."""
+    if not torch.compiler.is_compiling():
+        out = _native.gate_residual(x, gate, h)
+        if out is not None:
+            return out
     xp, xt = fwAD.unpack_dual(x)
     hp, ht = fwAD.unpack_dual(h)
     gp, gt = fwAD.unpack_dual(gate)

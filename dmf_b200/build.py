@@ -1,7 +1,8 @@
-"""Build the C-ABI shared library (dmf_b200/libdmf_attn.so) with nvcc for sm_100a.
+"""Build the C-ABI shared library (dmf_b200/libdmf_attn.so) with nvcc for sm_100a, and the native host path of the Python
+surface (dmf_b200/_dmf_torch.so, csrc/torch_host.cpp) with the C++ compiler.
 
-The library is built in-tree so that it travels with the source snapshot; it has
-no Python or torch dependency.  ``python -m dmf_b200.build`` builds it by hand.
+Both are built in-tree so that they travel with the source snapshot.  The library has no Python or torch dependency; the
+host module links it and torch.  ``python -m dmf_b200.build`` builds them by hand.
 """
 
 from __future__ import annotations
@@ -18,6 +19,9 @@ CSRC = PKG / "csrc"
 INCLUDE = PKG.parent / "include"
 LIB = PKG / "libdmf_attn.so"
 
+HOST_MODULE = PKG / "_dmf_torch.so"
+HOST_SOURCE = CSRC / "torch_host.cpp"
+
 SOURCES = ["dmf_attn.cu", "dmf_adaln.cu", "dmf_step.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -33,12 +37,16 @@ def find_nvcc() -> str | None:
     return cand if cand and Path(cand).exists() else None
 
 
+def _older(target: Path, deps) -> bool:
+    return not target.exists() or any(d.stat().st_mtime > target.stat().st_mtime for d in deps)
+
+
 def _stale() -> bool:
-    if not LIB.exists():
-        return True
-    t = LIB.stat().st_mtime
-    deps = list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cuh")) + list(INCLUDE.glob("*.h"))
-    return any(d.stat().st_mtime > t for d in deps)
+    return _older(LIB, [*CSRC.glob("*.cu"), *CSRC.glob("*.cuh"), *INCLUDE.glob("*.h")])
+
+
+def _host_stale() -> bool:
+    return _older(HOST_MODULE, [HOST_SOURCE, *(CSRC / "compat").rglob("*.hpp"), *INCLUDE.glob("*.h")])
 
 
 def build(force: bool = False, verbose: bool = False) -> Path:
@@ -76,5 +84,41 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     return LIB
 
 
+def build_host(force: bool = False) -> Path:
+    """Compile the native host path (torch_host.cpp) if it is missing or older than its sources; same locking as build()."""
+    lib = build()
+    if not force and not _host_stale():
+        return HOST_MODULE
+    import sysconfig
+
+    import torch
+    root = Path(torch.__file__).resolve().parent
+    nvcc = find_nvcc()
+    if nvcc is None:
+        raise RuntimeError("no CUDA toolkit: cannot build dmf_b200/_dmf_torch.so")
+    with open(PKG / ".build.lock", "w") as lock:
+        fcntl.flock(lock, fcntl.LOCK_EX)
+        try:
+            if not force and not _host_stale():
+                return HOST_MODULE
+            tmp = HOST_MODULE.with_name(f".{HOST_MODULE.name}.{os.getpid()}.tmp")
+            includes = [root / "include", root / "include" / "torch" / "csrc" / "api" / "include",
+                        sysconfig.get_paths()["include"], Path(nvcc).resolve().parent.parent / "include", CSRC / "compat"]
+            cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+                   "-DTORCH_EXTENSION_NAME=_dmf_torch", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
+                   *(f"-isystem{i}" for i in includes), f"-I{INCLUDE}", str(HOST_SOURCE), "-o", str(tmp), f"-L{root / 'lib'}",
+                   "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda", "-ltorch_python",
+                   f"-L{lib.parent}", f"-l:{lib.name}", "-Wl,-rpath,$ORIGIN"]
+            res = subprocess.run(cmd, capture_output=True, text=True)
+            if res.returncode != 0:
+                tmp.unlink(missing_ok=True)
+                raise RuntimeError(f"{cmd[0]} failed ({res.returncode}):\n{res.stdout}\n{res.stderr}")
+            os.replace(tmp, HOST_MODULE)
+        finally:
+            fcntl.flock(lock, fcntl.LOCK_UN)
+    return HOST_MODULE
+
+
 if __name__ == "__main__":
     print(build(force="--force" in sys.argv, verbose="-v" in sys.argv))
+    print(build_host(force="--force" in sys.argv))

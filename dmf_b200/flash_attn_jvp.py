@@ -27,7 +27,7 @@ from __future__ import annotations
 import torch
 import torch.autograd.forward_ad as fwAD
 
-from . import ops
+from . import _native, ops
 
 
 class FlashAttnFunc(torch.autograd.Function):
@@ -80,6 +80,10 @@ def _is_dual_mode(*tensors):
 
 
 def flash_attn_func(q, k, v, softmax_scale=None):
+    if not torch.compiler.is_compiling():
+        out = _native.attn_func(q, k, v, softmax_scale)
+        if out is not None:
+            return out
     if _is_dual_mode(q, k, v):
         primals, tangents = [], []
         for tensor in (q, k, v):
@@ -131,6 +135,10 @@ class FlashAttnQKVPackedFunc(torch.autograd.Function):
 def flash_attn_qkvpacked_func(qkv, softmax_scale=None):
     if qkv.dim() != 5 or qkv.shape[2] != 3:
         raise ValueError("expected a (B, L, 3, H, D) tensor")
+    if not torch.compiler.is_compiling():
+        out = _native.attn_qkvpacked(qkv, softmax_scale)
+        if out is not None:
+            return out
     primal, tangent = fwAD.unpack_dual(qkv)
     if tangent is not None:
         out, _, t_out = FlashAttnQKVPackedFunc.apply(primal, tangent, softmax_scale)

@@ -16,22 +16,39 @@ register_fake does (models/flash_attention_2_jvp.py:64-88, 143-174).
 from __future__ import annotations
 
 import ctypes as C
-import os
+import sys
+import types
 from typing import Tuple
 
 import torch
 
-from . import _lib
+from . import _lib, _native
 
 _DTYPES = {torch.bfloat16: _lib.BF16, torch.float16: _lib.FP16}
 
-# Kernel launches made through this module since import (a backward call launches two kernels).
-launch_count = 0
+class _Module(types.ModuleType):
+    """``ops.launch_count``: kernel launches of this package since import (a backward call counts two).  The counter lives
+    in the native host path, which makes most of them."""
+
+    @property
+    def launch_count(self) -> int:
+        return _native.launch_count()
+
+    @launch_count.setter
+    def launch_count(self, n: int) -> None:
+        _native.set_launch_count(n)
+
+
+sys.modules[__name__].__class__ = _Module
+
+
+def _count(n: int) -> None:
+    _native.set_launch_count(_native.launch_count() + n)
+
 
 # One int32 per device that kernels write to when a device-side wait runs out.
 _status_words: dict[int, torch.Tensor] = {}
-# DMF_ATTN_CHECK=1 reads the status word back after every call (synchronises; for tests and debugging).
-_CHECK_EVERY_CALL = os.environ.get("DMF_ATTN_CHECK", "0") == "1"
+_CHECK_EVERY_CALL = _native.CHECK_EVERY_CALL
 
 
 def _status_word(device: torch.device) -> torch.Tensor:
@@ -40,6 +57,7 @@ def _status_word(device: torch.device) -> torch.Tensor:
     if w is None:
         w = torch.zeros(1, dtype=torch.int32, device=device)
         _status_words[idx] = w
+        _native.set_status_word(idx, w.data_ptr())
     return w
 
 
@@ -135,8 +153,7 @@ def fwd_dual_raw(q, k, v, tq, tk, tv, scale: float):
         a.q, a.k, a.v, a.tq, a.tk, a.tv, a.o, a.to = (_t4(x) for x in (q, k, v, tq, tk, tv, o, to))
         a.lse = lse.data_ptr()
         _lib.check(_lib.load().dmf_attn_fwd_dual(C.byref(a)))
-        global launch_count
-        launch_count += 1
+        _count(1)
         if _CHECK_EVERY_CALL:
             check_device_status(q.device)
     return o, to, lse
@@ -156,8 +173,7 @@ def fwd_raw(q, k, v, scale: float):
         a.q, a.k, a.v, a.o = (_t4(x) for x in (q, k, v, o))
         a.lse = lse.data_ptr()
         _lib.check(_lib.load().dmf_attn_fwd(C.byref(a)))
-        global launch_count
-        launch_count += 1
+        _count(1)
         if _CHECK_EVERY_CALL:
             check_device_status(q.device)
     return o, lse
@@ -190,8 +206,7 @@ def bwd_raw(dout, q, k, v, o, lse, scale: float, packed_out: bool = False):
         a.lse = lse.data_ptr()
         a.workspace, a.workspace_bytes = ws.data_ptr(), ws_bytes
         _lib.check(lib.dmf_attn_bwd(C.byref(a)))
-        global launch_count
-        launch_count += 2
+        _count(2)
         if _CHECK_EVERY_CALL:
             check_device_status(q.device)
     return dqkv if packed_out else (dq, dk, dv)
@@ -278,8 +293,7 @@ def rmsnorm_fwd_raw(x, tx, weight, eps: float):
         a.weight = w.data_ptr()
         a.stream = torch.cuda.current_stream(x.device).cuda_stream
         _lib.check(_lib.load().dmf_rmsnorm_fwd(C.byref(a)))
-        global launch_count
-        launch_count += 1
+        _count(1)
     return y, ty
 
 
@@ -304,8 +318,7 @@ def rmsnorm_bwd_raw(dy, x, weight, eps: float):
         a.workspace, a.workspace_bytes = ws.data_ptr(), nbytes
         a.stream = torch.cuda.current_stream(x.device).cuda_stream
         _lib.check(lib.dmf_rmsnorm_bwd(C.byref(a)))
-        global launch_count
-        launch_count += 2
+        _count(2)
     return dx, dw
 
 

@@ -21,6 +21,7 @@ from __future__ import annotations
 import torch
 import torch.autograd.forward_ad as fwAD
 
+from . import _native
 from . import ops  # noqa: F401  (registers the custom ops)
 
 
@@ -58,6 +59,10 @@ class RmsNormFunc(torch.autograd.Function):
 
 def rms_norm(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-6) -> torch.Tensor:
     """RMSNorm over the last dim of a (B, L, H, D) tensor; a dual tensor in gives a dual tensor out."""
+    if not torch.compiler.is_compiling():
+        out = _native.rms_norm(x, weight, eps)
+        if out is not None:
+            return out
     primal, tangent = fwAD.unpack_dual(x)
     if tangent is not None:
         w, _ = fwAD.unpack_dual(weight)
