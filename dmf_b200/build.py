@@ -22,7 +22,7 @@ LIB = PKG / "libdmf_attn.so"
 HOST_MODULE = PKG / "_dmf_torch.so"
 HOST_SOURCE = CSRC / "torch_host.cpp"
 
-SOURCES = ["dmf_attn.cu", "dmf_adaln.cu", "dmf_step.cu"]
+SOURCES = ["dmf_attn.cu", "attn_fwd_duo.cu", "dmf_adaln.cu", "dmf_step.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-lineinfo", "-O3", "-std=c++17",
@@ -42,7 +42,7 @@ def _older(target: Path, deps) -> bool:
 
 
 def _stale() -> bool:
-    return _older(LIB, [*CSRC.glob("*.cu"), *CSRC.glob("*.cuh"), *INCLUDE.glob("*.h")])
+    return _older(LIB, [*CSRC.glob("*.cu"), *CSRC.glob("*.cuh"), *CSRC.glob("*.h"), *INCLUDE.glob("*.h")])
 
 
 def _host_stale() -> bool:

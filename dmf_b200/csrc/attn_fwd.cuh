@@ -72,6 +72,7 @@ struct FwdParams {
   int32_t* status_word;
   int batch, heads, seqlen_q, seqlen_kv, head_dim;
   int num_q_tiles, num_tiles;
+  int unit_tiles;  // attn_fwd_duo_kernel: query tiles of one unit of work
   float scale, scale_log2e;
   // Sector alignment of head rows (only used for head_dim 72, whose rows are 4.5 sectors of 32 B):
   // a row of (b, h) starts (align0 + b * align_b + h * align_h) mod 32 bytes into a sector.  When

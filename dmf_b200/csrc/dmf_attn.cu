@@ -18,6 +18,7 @@
 #include "attn_bwd_stream.cuh"
 #include "attn_fwd.cuh"
 #include "attn_fwd_pair.cuh"
+#include "attn_launch.h"
 #include "rmsnorm.cuh"
 
 namespace {
@@ -176,10 +177,8 @@ template <typename T, int TAIL, bool kDual>
 int launch_fwd_inst(const FwdParams& p, int grid, cudaStream_t stream) {
   using TR = FwdTraits<TAIL, kDual>;
   auto kernel = attn_fwd_kernel<T, TAIL, kDual>;
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TR::kSmemBytes) != cudaSuccess) {
-    (void)cudaGetLastError();
-    return DMF_ATTN_ERR_LAUNCH;
-  }
+  static bool done[64];
+  if (!allow_smem(kernel, TR::kSmemBytes, done)) return DMF_ATTN_ERR_LAUNCH;
   kernel<<<grid, kFwdThreads, TR::kSmemBytes, stream>>>(p);
   return cudaGetLastError() == cudaSuccess ? DMF_ATTN_OK : DMF_ATTN_ERR_LAUNCH;
 }
@@ -195,16 +194,14 @@ int launch_fwd_tail(const FwdParams& p, int tail, int grid, cudaStream_t stream)
   }
 }
 
-// ---- forward launch, CTA-pair variant (dual pass, head_dim <= 96, even number of query tiles) ----
+// ---- dual forward launch, CTA-pair variant (head_dim <= 96, even number of query tiles) ----
 
-template <typename T, int TAIL, bool kDual, bool kShort, bool kF32Out = false>
+template <typename T, int TAIL, bool kShort, bool kF32Out = false>
 int launch_pair_inst(const FwdParams& p, int clusters, cudaStream_t stream) {
   using TR = PairTraits<TAIL, kShort>;
-  auto kernel = attn_fwd_pair_kernel<T, TAIL, kDual, kShort, kF32Out>;
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TR::kSmemBytes) != cudaSuccess) {
-    (void)cudaGetLastError();
-    return DMF_ATTN_ERR_LAUNCH;
-  }
+  auto kernel = attn_fwd_pair_kernel<T, TAIL, kShort, kF32Out>;
+  static bool done[64];
+  if (!allow_smem(kernel, TR::kSmemBytes, done)) return DMF_ATTN_ERR_LAUNCH;
   cudaLaunchConfig_t cfg;
   std::memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = dim3(2 * clusters, 1, 1);
@@ -218,7 +215,8 @@ int launch_pair_inst(const FwdParams& p, int clusters, cudaStream_t stream) {
   attr.val.clusterDim.z = 1;
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
-  if (std::getenv("DMF_ATTN_DEBUG") != nullptr) {
+  static const bool debug = std::getenv("DMF_ATTN_DEBUG") != nullptr;
+  if (debug) {
     int n = -1;
     cudaError_t e = cudaOccupancyMaxActiveClusters(&n, kernel, &cfg);
     std::fprintf(stderr, "[dmf_attn] pair kernel: %d clusters requested, max active clusters %d (%s)\n", clusters, n,
@@ -231,14 +229,14 @@ int launch_pair_inst(const FwdParams& p, int clusters, cudaStream_t stream) {
   return DMF_ATTN_OK;
 }
 
-template <typename T, bool kDual>
+template <typename T>
 int launch_pair_tail(const FwdParams& p, int tail, int clusters, cudaStream_t stream) {
   switch (tail) {
-    case 0: return launch_pair_inst<T, 0, kDual, false>(p, clusters, stream);
+    case 0: return launch_pair_inst<T, 0, false>(p, clusters, stream);
     case 16:  // the only head_dim whose shared-memory split depends on the length of the key sequence
-      return p.seqlen_kv <= kShortMaxBlocks * kBlockKV ? launch_pair_inst<T, 16, kDual, true>(p, clusters, stream)
-                                                       : launch_pair_inst<T, 16, kDual, false>(p, clusters, stream);
-    case 32: return launch_pair_inst<T, 32, kDual, false>(p, clusters, stream);
+      return p.seqlen_kv <= kShortMaxBlocks * kBlockKV ? launch_pair_inst<T, 16, true>(p, clusters, stream)
+                                                       : launch_pair_inst<T, 16, false>(p, clusters, stream);
+    case 32: return launch_pair_inst<T, 32, false>(p, clusters, stream);
     default: return DMF_ATTN_ERR_HEAD_DIM;
   }
 }
@@ -247,10 +245,10 @@ int launch_pair_tail(const FwdParams& p, int tail, int clusters, cudaStream_t st
 int launch_pair_f32out(const FwdParams& p, int tail, int clusters, cudaStream_t stream) {
   const bool is_short = p.seqlen_kv <= kShortMaxBlocks * kBlockKV;
   switch (tail) {
-    case 0: return launch_pair_inst<__nv_bfloat16, 0, true, false, true>(p, clusters, stream);
+    case 0: return launch_pair_inst<__nv_bfloat16, 0, false, true>(p, clusters, stream);
     case 16:
-      return is_short ? launch_pair_inst<__nv_bfloat16, 16, true, true, true>(p, clusters, stream)
-                      : launch_pair_inst<__nv_bfloat16, 16, true, false, true>(p, clusters, stream);
+      return is_short ? launch_pair_inst<__nv_bfloat16, 16, true, true>(p, clusters, stream)
+                      : launch_pair_inst<__nv_bfloat16, 16, false, true>(p, clusters, stream);
     default: return DMF_ATTN_ERR_HEAD_DIM;
   }
 }
@@ -265,9 +263,14 @@ bool pair_kernel_enabled() {
 }
 
 // Which kernel template the launcher picks for a problem; one rule for the launch and for dmf_attn_kernel_name.
-bool fwd_uses_pair(int tail, int seqlen_q) {
-  return tail >= 0 && tail <= 32 && ((seqlen_q / kBlockQ) % 2 == 0) && pair_kernel_enabled();
+bool fwd_uses_pair(bool dual, int tail, int seqlen_q) {
+  return dual && tail >= 0 && tail <= 32 && ((seqlen_q / kBlockQ) % 2 == 0) && pair_kernel_enabled();
 }
+
+// The plain forward takes two query tiles per CTA wherever a head has two.  With one (128 query rows) half of that kernel
+// would idle: the single-CTA kernel, whose two warpgroups share a tile, does 512 x 16 heads x 128 tokens in 124 us
+// instead of 164.
+bool fwd_uses_duo(bool dual, int seqlen_q) { return !dual && seqlen_q >= 2 * kBlockQ; }
 
 int run_fwd(const dmf_attn_fwd_args* a, bool dual, bool f32out = false) {
   int st = validate_fwd(a, dual, f32out ? 4 : 2);
@@ -281,8 +284,9 @@ int run_fwd(const dmf_attn_fwd_args* a, bool dual, bool f32out = false) {
   const int B = a->batch, H = a->heads, D = a->head_dim, Lq = a->seqlen_q, Lk = a->seqlen_kv, dt = a->dtype;
   if ((st = make_map_pair(&p.q_main, &p.q_tail, a->q, dt, B, Lq, H, D, tail, kBlockQ)) != DMF_ATTN_OK) return st;
   // CTA-pair kernel: dual pass, P in its own tensor-memory columns (head_dim <= 96), tiles pair up
-  const bool pair = fwd_uses_pair(tail, Lq);
-  if (f32out && !(pair && dual && dt == DMF_ATTN_BF16 && tail <= 16)) return DMF_ATTN_ERR_HEAD_DIM;
+  const bool duo = fwd_uses_duo(dual, Lq);
+  const bool pair = fwd_uses_pair(dual, tail, Lq);
+  if (f32out && !(pair && dt == DMF_ATTN_BF16 && tail <= 16)) return DMF_ATTN_ERR_HEAD_DIM;
   const int k_box_rows = pair ? kBlockKV / 2 : kBlockKV;  // a CTA of a pair loads half of the key rows
   if ((st = make_map_pair(&p.k_main, &p.k_tail, a->k, dt, B, Lk, H, D, tail, k_box_rows)) != DMF_ATTN_OK) return st;
   if ((st = make_map(&p.v_map, a->v, dt, B, Lk, H, D, 32, kBlockKV, CU_TENSOR_MAP_SWIZZLE_64B)) != DMF_ATTN_OK) return st;
@@ -333,8 +337,14 @@ int run_fwd(const dmf_attn_fwd_args* a, bool dual, bool f32out = false) {
   if ((pair || !dual) && !f32out) {  // kernels that write their outputs with TMA stores
     if ((st = make_map_pair(&p.o_main, &p.o_tail, a->o, dt, B, Lq, H, D, tail, kBlockQ)) != DMF_ATTN_OK) return st;
   }
+  if (duo) {
+    // one tile per CTA where that fills no more than the GPU: the call's latency is one tile's chain either way
+    p.unit_tiles = p.num_tiles <= sm_count ? 1 : 2;
+    p.num_tiles = B * H * ((p.num_q_tiles + p.unit_tiles - 1) / p.unit_tiles);
+    return launch_fwd_duo(p, tail, dt, p.num_tiles < sm_count ? p.num_tiles : sm_count, stream);
+  }
   if (pair) {
-    if (dual && !f32out &&
+    if (!f32out &&
         (st = make_map_pair(&p.to_main, &p.to_tail, a->to, dt, B, Lq, H, D, tail, kBlockQ)) != DMF_ATTN_OK)
       return st;
     p.align_enable[1] = 0;  // the pair kernel's V column order has no room for the 8-column shift
@@ -342,11 +352,8 @@ int run_fwd(const dmf_attn_fwd_args* a, bool dual, bool f32out = false) {
     const int max_clusters = sm_count / 2;
     const int clusters = p.num_tiles < max_clusters ? p.num_tiles : max_clusters;
     if (f32out) return launch_pair_f32out(p, tail, clusters, stream);
-    if (dual)
-      return dt == DMF_ATTN_BF16 ? launch_pair_tail<__nv_bfloat16, true>(p, tail, clusters, stream)
-                                 : launch_pair_tail<__half, true>(p, tail, clusters, stream);
-    return dt == DMF_ATTN_BF16 ? launch_pair_tail<__nv_bfloat16, false>(p, tail, clusters, stream)
-                               : launch_pair_tail<__half, false>(p, tail, clusters, stream);
+    return dt == DMF_ATTN_BF16 ? launch_pair_tail<__nv_bfloat16>(p, tail, clusters, stream)
+                               : launch_pair_tail<__half>(p, tail, clusters, stream);
   }
   const int grid = p.num_tiles < sm_count ? p.num_tiles : sm_count;
   if (dt == DMF_ATTN_BF16)
@@ -400,10 +407,8 @@ template <typename T, int TAIL, int kMode>
 int launch_bwd_inst(const BwdParams& p, int grid, cudaStream_t stream) {
   using TR = BwdTraits<TAIL>;
   auto kernel = attn_bwd_kernel<T, TAIL, kMode>;
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TR::kSmemBytes) != cudaSuccess) {
-    (void)cudaGetLastError();
-    return DMF_ATTN_ERR_LAUNCH;
-  }
+  static bool done[64];
+  if (!allow_smem(kernel, TR::kSmemBytes, done)) return DMF_ATTN_ERR_LAUNCH;
   kernel<<<grid, kBwdThreads, TR::kSmemBytes, stream>>>(p);
   return cudaGetLastError() == cudaSuccess ? DMF_ATTN_OK : DMF_ATTN_ERR_LAUNCH;
 }
@@ -413,10 +418,8 @@ template <typename T, int TAIL, int kMode>
 int launch_bwd_split_inst(const BwdParams& p, int grid, cudaStream_t stream) {
   using TR = BwdSplitTraits<TAIL>;
   auto kernel = attn_bwd_split_kernel<T, TAIL, kMode>;
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TR::kSmemBytes) != cudaSuccess) {
-    (void)cudaGetLastError();
-    return DMF_ATTN_ERR_LAUNCH;
-  }
+  static bool done[64];
+  if (!allow_smem(kernel, TR::kSmemBytes, done)) return DMF_ATTN_ERR_LAUNCH;
   kernel<<<grid, kBwdSplitThreads, TR::kSmemBytes, stream>>>(p);
   return cudaGetLastError() == cudaSuccess ? DMF_ATTN_OK : DMF_ATTN_ERR_LAUNCH;
 }
@@ -469,10 +472,8 @@ template <typename T, int TAIL>
 int launch_bwd_fused_inst(const BwdFusedParams& p, int clusters, cudaStream_t stream) {
   using TR = BwdFusedTraits<TAIL>;
   auto kernel = attn_bwd_fused_kernel<T, TAIL>;
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TR::kSmemBytes) != cudaSuccess) {
-    (void)cudaGetLastError();
-    return DMF_ATTN_ERR_LAUNCH;
-  }
+  static bool done[64];
+  if (!allow_smem(kernel, TR::kSmemBytes, done)) return DMF_ATTN_ERR_LAUNCH;
   cudaLaunchConfig_t cfg;
   std::memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = dim3(2 * clusters, 1, 1);
@@ -544,11 +545,8 @@ int launch_bwd_stream_inst(const BwdStreamParams& p, const dmf_attn_bwd_args* a,
   auto kernel = attn_bwd_stream_kernel<T, TAIL>;
   auto convert = bwd_dq_convert_kernel<T>;
   const int convert_smem = (p.head_dim / 4) * 128 * 16;
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TR::kSmemBytes) != cudaSuccess ||
-      cudaFuncSetAttribute(convert, cudaFuncAttributeMaxDynamicSharedMemorySize, convert_smem) != cudaSuccess) {
-    (void)cudaGetLastError();
-    return DMF_ATTN_ERR_LAUNCH;
-  }
+  static bool done[64], convert_done[64];
+  if (!allow_smem(kernel, TR::kSmemBytes, done) || !allow_smem(convert, 32 * 128 * 16, convert_done)) return DMF_ATTN_ERR_LAUNCH;
   // rows of the pre-kernel's block: 32 positions of all heads, fewer when that does not fit 48 KB of shared memory
   int lrows = 32;
   while (lrows > 1 && static_cast<size_t>(lrows) * p.heads * (p.head_dim / 8) * sizeof(float) > 48 * 1024) lrows /= 2;
@@ -817,7 +815,9 @@ int kernel_name(int op, int seqlen_q, int seqlen_kv, int head_dim, int dtype, ch
   const char* t = dtype == DMF_ATTN_BF16 ? "bf16" : "fp16";
   if (op == 0 || op == 1) {
     const char* kind = op == 0 ? "dual" : "plain";
-    if (fwd_uses_pair(tail, seqlen_q)) {
+    if (fwd_uses_duo(op == 0, seqlen_q)) {
+      std::snprintf(buf, len, "attn_fwd_duo_kernel<%s, TAIL=%d> (two query tiles per CTA)", t, tail);
+    } else if (fwd_uses_pair(op == 0, tail, seqlen_q)) {
       const bool is_short = tail == 16 && seqlen_kv <= kShortMaxBlocks * kBlockKV;
       std::snprintf(buf, len, "attn_fwd_pair_kernel<%s, TAIL=%d, %s%s> (cta_group::2 cluster pair)", t, tail, kind,
                     is_short ? ", short" : "");

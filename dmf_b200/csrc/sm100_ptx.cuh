@@ -72,7 +72,7 @@ constexpr long long kWaitLimitCycles = 4000000000ll;
 // when its own wait ran out; every other wait then returns false promptly.
 // The first poll is inlined (a wait that is already satisfied costs one shared-memory
 // round trip); everything else lives in an out-of-line slow path.
-__device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, volatile int* abort_flag,
+static __device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, volatile int* abort_flag,
                                             int32_t* status_word, int32_t code,
                                             long long limit_cycles = kWaitLimitCycles) {
   uint32_t spins = 0;

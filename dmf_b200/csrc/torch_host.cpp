@@ -162,6 +162,17 @@ int attn_dtype(at::ScalarType t) {
 
 dmf_attn_tensor t4(const Tensor& x) { return {x.data_ptr(), x.stride(0), x.stride(1), x.stride(2)}; }
 
+// slice i of a (B, L, 3, H, D) tensor
+dmf_attn_tensor t4_packed(const Tensor& x, int i) {
+  return {static_cast<char*>(x.data_ptr()) + i * x.stride(2) * static_cast<int64_t>(x.element_size()), x.stride(0), x.stride(1), x.stride(3)};
+}
+
+// the slices of a packed tensor can be read (and written) where they are
+bool packed_ok(const Tensor& x) {
+  return x.stride(4) == 1 && reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 == 0 && x.stride(0) % 8 == 0 && x.stride(1) % 8 == 0 &&
+         x.stride(2) % 8 == 0 && x.stride(3) % 8 == 0;
+}
+
 // unit stride on D, 16-byte aligned base and strides (maybe_contiguous, models/flash_attention_2_jvp.py:24-25)
 Tensor prep(const Tensor& x) {
   if (x.stride(3) == 1 && reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 == 0) {
@@ -188,70 +199,97 @@ struct AttnOut {
   int status = DMF_ATTN_OK;
 };
 
-AttnOut attn_forward(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor* tq_, const Tensor* tk_,
-                     const Tensor* tv_, double scale) {
-  const c10::cuda::CUDAGuard device_guard(q_.device());
-  const bool dual = tq_ != nullptr;
-  const Tensor q = prep(q_), k = prep(k_), v = prep(v_);
+template <typename A>
+void attn_sizes(A* a, const Tensor& q, int64_t B, int64_t L, int64_t Lk, int64_t H, int64_t D, double scale) {
+  a->batch = B; a->seqlen_q = L; a->seqlen_kv = Lk; a->heads = H; a->head_dim = D;
+  a->dtype = attn_dtype(q.scalar_type());
+  a->softmax_scale = static_cast<float>(scale);
+  a->status_word = g_status_word[q.get_device()].load(std::memory_order_acquire);
+  a->stream = c10::cuda::getCurrentCUDAStream(q.get_device()).stream();
+}
+
+// outputs and launch, with the inputs of `a` filled in
+AttnOut attn_launch(dmf_attn_fwd_args* a, const Tensor& like, bool dual) {
   AttnOut r;
-  const int64_t B = q.size(0), L = q.size(1), H = q.size(2), D = q.size(3);
-  r.o = at::empty({B, L, H, D}, q.options());
-  r.lse = at::empty({B, H, L}, q.options().dtype(at::kFloat));
-  dmf_attn_fwd_args a = {};
-  a.batch = B; a.seqlen_q = L; a.seqlen_kv = k.size(1); a.heads = H; a.head_dim = D;
-  a.dtype = attn_dtype(q.scalar_type());
-  a.softmax_scale = static_cast<float>(scale);
-  a.q = t4(q); a.k = t4(k); a.v = t4(v); a.o = t4(r.o);
-  a.lse = r.lse.data_ptr<float>();
-  a.status_word = g_status_word[q.get_device()].load(std::memory_order_acquire);
-  a.stream = c10::cuda::getCurrentCUDAStream(q.get_device()).stream();
+  const int64_t B = a->batch, L = a->seqlen_q, H = a->heads, D = a->head_dim;
+  r.o = at::empty({B, L, H, D}, like.options());
+  r.lse = at::empty({B, H, L}, like.options().dtype(at::kFloat));
+  a->o = t4(r.o);
+  a->lse = r.lse.data_ptr<float>();
   if (dual) {
-    const Tensor tq = prep(*tq_), tk = prep(*tk_), tv = prep(*tv_);
-    r.to = at::empty({B, L, H, D}, q.options());
-    a.tq = t4(tq); a.tk = t4(tk); a.tv = t4(tv); a.to = t4(r.to);
-    r.status = dmf_attn_fwd_dual(&a);
-  } else {
-    r.status = dmf_attn_fwd(&a);
+    r.to = at::empty({B, L, H, D}, like.options());
+    a->to = t4(r.to);
   }
+  r.status = dual ? dmf_attn_fwd_dual(a) : dmf_attn_fwd(a);
   if (r.status == DMF_ATTN_OK) g_launches.fetch_add(1, std::memory_order_relaxed);
   return r;
 }
 
-// dq, dk, dv, or with `packed` one (B, L, 3, H, D) gradient
-variable_list attn_backward(const Tensor& dout_, const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& o_,
-                            const Tensor& lse, double scale, bool packed) {
+AttnOut attn_forward(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor* tq_, const Tensor* tk_,
+                     const Tensor* tv_, double scale) {
   const c10::cuda::CUDAGuard device_guard(q_.device());
-  TORCH_CHECK(same_kind(q_, dout_) && dout_.sizes() == o_.sizes(), "dmf_b200 attention backward: unexpected gradient");
-  const Tensor dout = prep(dout_), q = prep(q_), k = prep(k_), v = prep(v_), o = prep(o_);
-  const int64_t B = q.size(0), L = q.size(1), H = q.size(2), D = q.size(3), Lk = k.size(1);
-  variable_list grads;
-  Tensor dq, dk, dv;
-  if (packed) {
-    grads = {at::empty({B, L, 3, H, D}, q.options())};
-    dq = grads[0].select(2, 0); dk = grads[0].select(2, 1); dv = grads[0].select(2, 2);
-  } else {
-    dq = at::empty({B, L, H, D}, q.options());
-    dk = at::empty({B, Lk, H, D}, q.options());
-    dv = at::empty({B, Lk, H, D}, q.options());
-    grads = {dq, dk, dv};
-  }
-  const size_t bytes = dmf_attn_bwd_workspace_bytes(B, L, Lk, H, D);
-  const Tensor ws = at::empty({static_cast<int64_t>(std::max<size_t>(bytes, 16))}, q.options().dtype(at::kByte));
-  dmf_attn_bwd_args a = {};
-  a.batch = B; a.seqlen_q = L; a.seqlen_kv = Lk; a.heads = H; a.head_dim = D;
-  a.dtype = attn_dtype(q.scalar_type());
-  a.softmax_scale = static_cast<float>(scale);
-  a.dout = t4(dout); a.q = t4(q); a.k = t4(k); a.v = t4(v); a.o = t4(o);
-  a.lse = lse.data_ptr<float>();
-  a.dq = t4(dq); a.dk = t4(dk); a.dv = t4(dv);
-  a.workspace = ws.data_ptr();
-  a.workspace_bytes = bytes;
-  a.status_word = g_status_word[q.get_device()].load(std::memory_order_acquire);
-  a.stream = c10::cuda::getCurrentCUDAStream(q.get_device()).stream();
-  const int st = dmf_attn_bwd(&a);
+  const Tensor q = prep(q_), k = prep(k_), v = prep(v_);
+  dmf_attn_fwd_args a = {};
+  attn_sizes(&a, q, q.size(0), q.size(1), k.size(1), q.size(2), q.size(3), scale);
+  a.q = t4(q); a.k = t4(k); a.v = t4(v);
+  if (tq_ == nullptr) return attn_launch(&a, q, false);
+  const Tensor tq = prep(*tq_), tk = prep(*tk_), tv = prep(*tv_);
+  a.tq = t4(tq); a.tk = t4(tk); a.tv = t4(tv);
+  return attn_launch(&a, q, true);
+}
+
+AttnOut attn_forward_packed(const Tensor& qkv_, const Tensor& tqkv_, double scale) {
+  const c10::cuda::CUDAGuard device_guard(qkv_.device());
+  const Tensor qkv = packed_ok(qkv_) ? qkv_ : qkv_.contiguous();
+  dmf_attn_fwd_args a = {};
+  attn_sizes(&a, qkv, qkv.size(0), qkv.size(1), qkv.size(1), qkv.size(3), qkv.size(4), scale);
+  a.q = t4_packed(qkv, 0); a.k = t4_packed(qkv, 1); a.v = t4_packed(qkv, 2);
+  if (!tqkv_.defined()) return attn_launch(&a, qkv, false);
+  const Tensor t = packed_ok(tqkv_) ? tqkv_ : tqkv_.contiguous();
+  a.tq = t4_packed(t, 0); a.tk = t4_packed(t, 1); a.tv = t4_packed(t, 2);
+  return attn_launch(&a, qkv, true);
+}
+
+// workspace and launch of a backward, with the tensors of `a` filled in
+void attn_launch_bwd(dmf_attn_bwd_args* a, const Tensor& like, const Tensor& lse) {
+  const size_t bytes = dmf_attn_bwd_workspace_bytes(a->batch, a->seqlen_q, a->seqlen_kv, a->heads, a->head_dim);
+  const Tensor ws = at::empty({static_cast<int64_t>(std::max<size_t>(bytes, 16))}, like.options().dtype(at::kByte));
+  a->lse = lse.data_ptr<float>();
+  a->workspace = ws.data_ptr();
+  a->workspace_bytes = bytes;
+  const int st = dmf_attn_bwd(a);
   TORCH_CHECK(st == DMF_ATTN_OK, "dmf_attn: ", dmf_attn_status_string(st));
   g_launches.fetch_add(2, std::memory_order_relaxed);
+}
+
+variable_list attn_backward(const Tensor& dout_, const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& o,
+                            const Tensor& lse, double scale) {
+  const c10::cuda::CUDAGuard device_guard(q_.device());
+  TORCH_CHECK(same_kind(q_, dout_) && dout_.sizes() == o.sizes(), "dmf_b200 attention backward: unexpected gradient");
+  const Tensor dout = prep(dout_), q = prep(q_), k = prep(k_), v = prep(v_);
+  variable_list grads = {at::empty(q.sizes(), q.options()), at::empty(k.sizes(), q.options()), at::empty(v.sizes(), q.options())};
+  dmf_attn_bwd_args a = {};
+  attn_sizes(&a, q, q.size(0), q.size(1), k.size(1), q.size(2), q.size(3), scale);
+  a.dout = t4(dout); a.q = t4(q); a.k = t4(k); a.v = t4(v); a.o = t4(o);
+  a.dq = t4(grads[0]); a.dk = t4(grads[1]); a.dv = t4(grads[2]);
+  attn_launch_bwd(&a, q, lse);
   return grads;
+}
+
+// one (B, L, 3, H, D) gradient
+Tensor attn_backward_packed(const Tensor& dout_, const Tensor& qkv_, const Tensor& o, const Tensor& lse, double scale) {
+  const c10::cuda::CUDAGuard device_guard(qkv_.device());
+  TORCH_CHECK(dout_.scalar_type() == o.scalar_type() && dout_.device() == o.device() && dout_.sizes() == o.sizes(),
+              "dmf_b200 attention backward: unexpected gradient");
+  const Tensor dout = prep(dout_), qkv = packed_ok(qkv_) ? qkv_ : qkv_.contiguous();
+  const Tensor grad = at::empty(qkv.sizes(), qkv.options());
+  dmf_attn_bwd_args a = {};
+  attn_sizes(&a, qkv, qkv.size(0), qkv.size(1), qkv.size(1), qkv.size(3), qkv.size(4), scale);
+  a.dout = t4(dout); a.o = t4(o);
+  a.q = t4_packed(qkv, 0); a.k = t4_packed(qkv, 1); a.v = t4_packed(qkv, 2);
+  a.dq = t4_packed(grad, 0); a.dk = t4_packed(grad, 1); a.dv = t4_packed(grad, 2);
+  attn_launch_bwd(&a, qkv, lse);
+  return grad;
 }
 
 struct RejectedError : std::exception {};  // the C ABI refused before any launch: the general route reports it
@@ -275,7 +313,7 @@ struct AttnNode : torch::autograd::Function<AttnNode> {
     if (!grads[0].defined()) {  // only the tangent output was used: it carries no gradient
       return {at::zeros_like(s[0]), at::zeros_like(s[1]), at::zeros_like(s[2]), Tensor(), Tensor(), Tensor(), Tensor()};
     }
-    variable_list g = attn_backward(grads[0], s[0], s[1], s[2], s[3], s[4], ctx->saved_data["scale"].toDouble(), false);
+    variable_list g = attn_backward(grads[0], s[0], s[1], s[2], s[3], s[4], ctx->saved_data["scale"].toDouble());
     g.resize(7);
     return g;
   }
@@ -284,25 +322,18 @@ struct AttnNode : torch::autograd::Function<AttnNode> {
 struct AttnPackedNode : torch::autograd::Function<AttnPackedNode> {
   static variable_list forward(AutogradContext* ctx, const Tensor& qkv, const std::optional<Tensor>& tqkv, double scale) {
     at::AutoDispatchBelowADInplaceOrView below_autograd;
-    const bool dual = tqkv.has_value();
-    Tensor t[3];
-    if (dual)
-      for (int i = 0; i < 3; ++i) t[i] = tqkv->select(2, i);
-    AttnOut r = attn_forward(qkv.select(2, 0), qkv.select(2, 1), qkv.select(2, 2), dual ? &t[0] : nullptr, &t[1], &t[2], scale);
+    AttnOut r = attn_forward_packed(qkv, value_of(tqkv), scale);
     if (r.status != DMF_ATTN_OK) throw RejectedError();
     ctx->save_for_backward({qkv, r.o, r.lse});
     ctx->saved_data["scale"] = scale;
     ctx->set_materialize_grads(false);
-    return dual ? variable_list{r.o, r.to} : variable_list{r.o};
+    return r.to.defined() ? variable_list{r.o, r.to} : variable_list{r.o};
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     at::AutoDispatchBelowADInplaceOrView below_autograd;
     const auto s = ctx->get_saved_variables();
     if (!grads[0].defined()) return {at::zeros_like(s[0]), Tensor(), Tensor()};
-    variable_list g = attn_backward(grads[0], s[0].select(2, 0), s[0].select(2, 1), s[0].select(2, 2), s[1], s[2],
-                                    ctx->saved_data["scale"].toDouble(), true);
-    g.resize(3);
-    return g;
+    return {attn_backward_packed(grads[0], s[0], s[1], s[2], ctx->saved_data["scale"].toDouble()), Tensor(), Tensor()};
   }
 };
 
@@ -362,10 +393,7 @@ std::optional<Tensor> attn_qkvpacked(const Tensor& qkv_, std::optional<double> s
     }
   } else {
     at::AutoDispatchBelowADInplaceOrView below_autograd;
-    Tensor t[3];
-    if (dual)
-      for (int i = 0; i < 3; ++i) t[i] = x.t.select(2, i);
-    AttnOut r = attn_forward(x.p.select(2, 0), x.p.select(2, 1), x.p.select(2, 2), dual ? &t[0] : nullptr, &t[1], &t[2], scale);
+    AttnOut r = attn_forward_packed(x.p, x.t, scale);
     if (r.status != DMF_ATTN_OK) return std::nullopt;
     o = r.o;
     to = r.to;

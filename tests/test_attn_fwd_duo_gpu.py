@@ -1,0 +1,32 @@
+"""The plain forward with two query tiles per CTA where it can go wrong: an odd tile count (the last unit of a head has one
+tile), one key block, single-tile units (a GPU that is not filled), several units per CTA, maxima that move late, every
+head-dim class; against the fp64 oracle, with the bf16 / fp16 rounding of P and of the result as the tolerance."""
+
+import pytest
+import torch
+
+from dmf_b200 import _lib
+from oracle import attn_jvp_oracle as orc
+from tests import _cabi
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.mark.parametrize("shape", [(1, 256, 128, 1, 64), (2, 384, 256, 3, 72), (40, 384, 128, 8, 72), (12, 640, 640, 7, 64),
+                                   (3, 256, 1152, 5, 80), (30, 384, 384, 4, 96), (24, 384, 256, 5, 128), (1, 2048, 2048, 2, 104)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_plain_forward_two_tiles_per_cta(shape, dtype):
+    B, Lq, Lk, H, D = shape
+    assert "duo" in _lib.kernel_name("fwd", Lq, Lk, D)
+    q = orc.make_inputs(B, Lq, H, D, seed=Lq + D)[0].to(dtype)
+    k, v = (x.to(dtype) for x in orc.make_inputs(B, Lk, H, D, seed=Lk + H)[1:3])
+    k = k * torch.linspace(0.5, 3.0, Lk).view(1, Lk, 1, 1).to(dtype)      # later blocks hold the larger logits
+    o, _, lse, _ = _cabi.fwd(*(x.to(DEV) for x in (q, k, v)))
+    assert not torch.isnan(o).any() and not torch.isnan(lse).any()
+    for b in {0, B // 2, B - 1}:
+        o_ref, lse_ref = orc.attn_fwd_closed_form(*[x[b:b + 1].float() for x in (q, k, v)])
+        # P and o are rounded to 8 (11) bits: 2^-9 (2^-12) relative each, independent over the keys
+        assert orc.rel_l2(o[b:b + 1].float().cpu(), o_ref) < (6e-3 if dtype == torch.bfloat16 else 1e-3)
+        # a quarter of the exponentials are cubics with 7.5e-5 relative error
+        assert float((lse[b:b + 1].cpu().double() - lse_ref).abs().max()) < 1e-4
