@@ -31,40 +31,43 @@ __device__ __forceinline__ void step_one(float& g, float& p, float& m, float& v,
   if (has_ema) e = e * a.ema_decay + p * (1.f - a.ema_decay);
 }
 
-// One thread handles one float4 of each buffer per iteration; all loads of an iteration are issued before the first
-// use.  kEma = false: no EMA buffer.  Grid-stride; the last (count % 4) elements are handled by thread 0 of block 0.
+// One thread, one float4 of each buffer; the last (count % 4) elements are handled by thread 0 of block 0.  HBM-bound, ten
+// streams of which five are written.  130M parameters with EMA, 5.2 GB: 834 us (6.24 TB/s, 0.96 of the measured copy rate);
+// with a grid-stride loop over 8 blocks per SM 845 us (a block that has finished is replaced at once, while a loop iteration
+// starts when its last store has issued), and with streaming hints on loads and stores on top 900 us.  Two vectors per thread:
+// 1105 us (fewer resident warps).
 template <bool kEma>
 __global__ void __launch_bounds__(256) step_tail_kernel(const StepParams a) {
   const float clip = a.grad_norm != nullptr ? fminf(1.f, a.max_grad_norm / (*a.grad_norm + 1e-6f)) : 1.f;
   const int64_t n4 = a.count >> 2;
-  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
   float4* g4 = reinterpret_cast<float4*>(a.grad);
   float4* p4 = reinterpret_cast<float4*>(a.param);
   float4* m4 = reinterpret_cast<float4*>(a.exp_avg);
   float4* v4 = reinterpret_cast<float4*>(a.exp_avg_sq);
   float4* e4 = reinterpret_cast<float4*>(a.ema);
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n4; i += stride) {
-    float4 g = __ldcs(g4 + i), p = __ldcs(p4 + i), m = __ldcs(m4 + i), v = __ldcs(v4 + i);
-    float4 e = kEma ? __ldcs(e4 + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+  const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i < n4) {
+    float4 g = g4[i], p = p4[i], m = m4[i], v = v4[i];
+    float4 e = kEma ? e4[i] : make_float4(0.f, 0.f, 0.f, 0.f);
     step_one(g.x, p.x, m.x, v.x, e.x, clip, kEma, a);
     step_one(g.y, p.y, m.y, v.y, e.y, clip, kEma, a);
     step_one(g.z, p.z, m.z, v.z, e.z, clip, kEma, a);
     step_one(g.w, p.w, m.w, v.w, e.w, clip, kEma, a);
-    __stcs(g4 + i, make_float4(0.f, 0.f, 0.f, 0.f));
-    p4[i] = p;  // the weights are read again right away by the next forward pass: keep them cacheable
-    __stcs(m4 + i, m);
-    __stcs(v4 + i, v);
-    if (kEma) __stcs(e4 + i, e);
+    g4[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    p4[i] = p;
+    m4[i] = m;
+    v4[i] = v;
+    if (kEma) e4[i] = e;
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
-    for (int64_t i = n4 << 2; i < a.count; ++i) {
-      float g = a.grad[i], p = a.param[i], m = a.exp_avg[i], v = a.exp_avg_sq[i], e = kEma ? a.ema[i] : 0.f;
+    for (int64_t k = n4 << 2; k < a.count; ++k) {
+      float g = a.grad[k], p = a.param[k], m = a.exp_avg[k], v = a.exp_avg_sq[k], e = kEma ? a.ema[k] : 0.f;
       step_one(g, p, m, v, e, clip, kEma, a);
-      a.grad[i] = 0.f;
-      a.param[i] = p;
-      a.exp_avg[i] = m;
-      a.exp_avg_sq[i] = v;
-      if (kEma) a.ema[i] = e;
+      a.grad[k] = 0.f;
+      a.param[k] = p;
+      a.exp_avg[k] = m;
+      a.exp_avg_sq[k] = v;
+      if (kEma) a.ema[k] = e;
     }
   }
 }
@@ -77,8 +80,8 @@ int run_step_tail(const dmf_step_tail_args* a) {
   for (const void* ptr : ptrs)
     if ((reinterpret_cast<uintptr_t>(ptr) & 15u) != 0) return DMF_ATTN_ERR_ALIGN;
   if (!(a->bias_correction2_sqrt > 0.f) || !(a->step_size == a->step_size)) return DMF_ATTN_ERR_SHAPE;
-  int dev = -1, sms = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+  int dev = -1;
+  if (cudaGetDevice(&dev) != cudaSuccess) {
     (void)cudaGetLastError();
     return DMF_ATTN_ERR_DEVICE;
   }
@@ -91,12 +94,11 @@ int run_step_tail(const dmf_step_tail_args* a) {
   p.ema_decay = a->ema_decay;
   const int64_t n4 = a->count >> 2;
   int64_t blocks = (n4 + 255) / 256;
-  const int64_t cap = static_cast<int64_t>(sms) * 8;  // 8 blocks of 256 threads per SM, grid-stride
-  if (blocks > cap) blocks = cap;
   if (blocks < 1) blocks = 1;
+  if (blocks > 0x7fffffff) return DMF_ATTN_ERR_SHAPE;  // 2^41 parameters
   cudaStream_t stream = static_cast<cudaStream_t>(a->stream);
-  if (a->ema != nullptr) step_tail_kernel<true><<<static_cast<int>(blocks), 256, 0, stream>>>(p);
-  else step_tail_kernel<false><<<static_cast<int>(blocks), 256, 0, stream>>>(p);
+  if (a->ema != nullptr) step_tail_kernel<true><<<static_cast<unsigned>(blocks), 256, 0, stream>>>(p);
+  else step_tail_kernel<false><<<static_cast<unsigned>(blocks), 256, 0, stream>>>(p);
   return cudaGetLastError() == cudaSuccess ? DMF_ATTN_OK : DMF_ATTN_ERR_LAUNCH;
 }
 
