@@ -207,6 +207,24 @@ int run_ln_modulate_bwd(const dmf_ln_modulate_bwd_args* a) {
   return launched();
 }
 
+// 8 channels at a time: 16-byte accesses to 16-bit rows need strides that are multiples of 8 (fp32 rows are read as two
+// 4-element vectors); every chunk of an adaLN projection of the model's widths has them.
+bool gate_vec8(const dmf_gate_residual_args* a, bool dual, bool tmod) {
+  auto rows = [](const dmf_rows& t, int dtype) { return dtype == DMF_ADALN_F32 || (t.stride_b % 8 == 0 && t.stride_l % 8 == 0); };
+  auto mod = [&](const dmf_mod& t) { return a->mod_dtype == DMF_ADALN_F32 || t.stride_b % 8 == 0; };
+  return a->channels % 8 == 0 && rows(a->x, a->wide_dtype) && rows(a->h, a->narrow_dtype) && rows(a->out, a->wide_dtype) &&
+         mod(a->gate) && (!tmod || mod(a->tgate)) &&
+         (!dual || (rows(a->tx, a->wide_dtype) && rows(a->th, a->narrow_dtype) && rows(a->tout, a->wide_dtype)));
+}
+
+// 16 rows per block (8 to 32 time the same), fewer where that leaves SMs without a few blocks, down to one row per thread
+int gate_rows_per_block(int batch, int seqlen, int lanes) {
+  constexpr int64_t kWantBlocks = 4 * 148;
+  int rpb = 16;
+  while (rpb > lanes && static_cast<int64_t>(batch) * ((seqlen + rpb - 1) / rpb) < kWantBlocks) rpb /= 2;
+  return rpb > lanes ? rpb : lanes;
+}
+
 int run_gate_residual_fwd(const dmf_gate_residual_args* a) {
   if (a == nullptr) return DMF_ATTN_ERR_NULL;
   int st;
@@ -237,13 +255,25 @@ int run_gate_residual_fwd(const dmf_gate_residual_args* a) {
   if (tmod) { p.tgate = a->tgate.ptr; p.tgate_sb = a->tgate.stride_b; }
   p.batch = a->batch; p.seqlen = a->seqlen; p.channels = a->channels;
   p.mod_f32 = a->mod_dtype == DMF_ADALN_F32;
-  const int grid = row_grid(static_cast<int64_t>(a->batch) * a->seqlen, sms);
   cudaStream_t stream = static_cast<cudaStream_t>(a->stream);
+  if (gate_vec8(a, dual, tmod)) {
+    const int nvec = a->channels / 8, threads = gate_row_threads(nvec) * gate_row_lanes(nvec);
+    p.rows_per_block = gate_rows_per_block(a->batch, a->seqlen, gate_row_lanes(nvec));
+    const dim3 grid((a->seqlen + p.rows_per_block - 1) / p.rows_per_block, a->batch);
+    return with_types(a->wide_dtype, a->narrow_dtype, [&](auto tw, auto tn) {
+      using TW = decltype(tw);
+      using TN = decltype(tn);
+      if (dual) gate_residual_fwd_kernel<TW, TN, true><<<grid, threads, 0, stream>>>(p);
+      else gate_residual_fwd_kernel<TW, TN, false><<<grid, threads, 0, stream>>>(p);
+      return launched();
+    });
+  }
+  const int grid = row_grid(static_cast<int64_t>(a->batch) * a->seqlen, sms);
   return with_types(a->wide_dtype, a->narrow_dtype, [&](auto tw, auto tn) {
     using TW = decltype(tw);
     using TN = decltype(tn);
-    if (dual) gate_residual_fwd_kernel<TW, TN, true><<<grid, kAdaThreads, 0, stream>>>(p);
-    else gate_residual_fwd_kernel<TW, TN, false><<<grid, kAdaThreads, 0, stream>>>(p);
+    if (dual) gate_residual_fwd_rows_kernel<TW, TN, true><<<grid, kAdaThreads, 0, stream>>>(p);
+    else gate_residual_fwd_rows_kernel<TW, TN, false><<<grid, kAdaThreads, 0, stream>>>(p);
     return launched();
   });
 }

@@ -182,3 +182,25 @@ def test_rejects_what_the_kernels_do_not_cover():
     with pytest.raises(RuntimeError):                                                               # width not compiled
         adaln.ln_modulate_fwd_raw(bad["x"], None, bad["shift"], bad["scale"], None, None, 1e-6, BF16)
     assert not adaln.usable(bad["x"]) and adaln.usable(g["x"], BF16) and not adaln.usable(c["x"])
+
+
+@pytest.mark.parametrize("wide,narrow", [(torch.float32, torch.float32), (torch.float32, torch.bfloat16),
+                                         (torch.bfloat16, torch.bfloat16)])
+@pytest.mark.parametrize("B,L,Cn", [(1, 1, 8), (3, 17, 136), (2, 33, 2056), (2, 9, 12), (5, 300, 384)])
+def test_gate_residual_forward_widths_and_row_counts(wide, narrow, B, L, Cn):
+    """8-channel and 4-channel kernels (C or a stride that is only a multiple of 4) against fp64."""
+    g = torch.Generator(device=DEV).manual_seed(B * L + Cn)
+    mk = lambda *s, dt: torch.randn(*s, device=DEV, generator=g).to(dt)
+    x, tx = mk(B, L, Cn, dt=wide), mk(B, L, Cn, dt=wide)
+    h, th = mk(B, L, Cn, dt=narrow), mk(B, L, Cn, dt=narrow)
+    padded = mk(B, L, Cn + 4, dt=narrow)
+    gate, tgate = mk(B, 1, Cn, dt=torch.bfloat16), mk(B, 1, Cn, dt=torch.bfloat16)
+    half = 2.0 ** -8 if wide == torch.bfloat16 else 2.0 ** -24
+    for hh in (h, padded[..., :Cn]):
+        out, tout = torch.func.jvp(adaln.gate_residual, (x, gate, hh), (tx, tgate, th))
+        assert torch.equal(adaln.gate_residual(x, gate, hh), out)
+        d = [t.double() for t in (x, gate, hh, tx, tgate, th)]
+        for got, terms in ((out, (d[0], d[1] * d[2])), (tout, (d[3], d[1] * d[5], d[4] * d[2]))):
+            # one rounding of the result (half a unit in the last place), and two of the fp32 sums of its terms
+            bound = 1.01 * half * sum(terms).abs() + 3 * 2.0 ** -24 * sum(t.abs() for t in terms)
+            assert bool(((got.double() - sum(terms)).abs() <= bound).all())
