@@ -29,7 +29,7 @@ EXPORTS = (
     "dmf_attn_fwd_dual_f32out", "dmf_attn_selftest_wait_limit", "dmf_attn_kernel_name",
     "dmf_rmsnorm_fwd", "dmf_rmsnorm_bwd", "dmf_rmsnorm_bwd_workspace_bytes",
     "dmf_ln_modulate_fwd", "dmf_ln_modulate_bwd", "dmf_adaln_bwd_workspace_bytes",
-    "dmf_gate_residual_fwd", "dmf_gate_residual_bwd",
+    "dmf_gate_residual_fwd", "dmf_gate_residual_bwd", "dmf_gelu",
     "dmf_step_tail",
 )
 ADALN_BF16, ADALN_F32 = 0, 2
@@ -127,6 +127,14 @@ class GateResidualBwdArgs(C.Structure):
     ]
 
 
+class GeluArgs(C.Structure):
+    """dmf_gelu_args (include/dmf_adaln.h)."""
+    _fields_ = [
+        ("count", C.c_int64), ("dtype", C.c_int32), ("reserved", C.c_int32),
+        ("x", C.c_void_p), ("t", C.c_void_p), ("y", C.c_void_p), ("ty", C.c_void_p), ("stream", C.c_void_p),
+    ]
+
+
 class StepTailArgs(C.Structure):
     """dmf_step_tail_args (include/dmf_step.h)."""
     _fields_ = [
@@ -194,7 +202,8 @@ def load() -> C.CDLL:
         lib.dmf_rmsnorm_bwd_workspace_bytes.restype = C.c_size_t
         lib.dmf_rmsnorm_bwd_workspace_bytes.argtypes = [C.c_int32]
         for name, args in (("dmf_ln_modulate_fwd", LnModulateArgs), ("dmf_ln_modulate_bwd", LnModulateBwdArgs),
-                           ("dmf_gate_residual_fwd", GateResidualArgs), ("dmf_gate_residual_bwd", GateResidualBwdArgs)):
+                           ("dmf_gate_residual_fwd", GateResidualArgs), ("dmf_gate_residual_bwd", GateResidualBwdArgs),
+                           ("dmf_gelu", GeluArgs)):
             fn = getattr(lib, name)
             fn.restype = C.c_int
             fn.argtypes = [C.POINTER(args)]

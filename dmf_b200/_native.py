@@ -28,7 +28,7 @@ launch_count, set_launch_count, set_status_word = _module.launch_count, _module.
 CHECK_EVERY_CALL = os.environ.get("DMF_ATTN_CHECK", "0") == "1"
 
 if CHECK_EVERY_CALL:
-    attn_func = attn_qkvpacked = rms_norm = ln_modulate = gate_residual = lambda *args: None
+    attn_func = attn_qkvpacked = rms_norm = ln_modulate = gate_residual = gelu = lambda *args: None
 else:
     attn_func, attn_qkvpacked = _module.attn_func, _module.attn_qkvpacked
-    rms_norm, ln_modulate, gate_residual = _module.rms_norm, _module.ln_modulate, _module.gate_residual
+    rms_norm, ln_modulate, gate_residual, gelu = _module.rms_norm, _module.ln_modulate, _module.gate_residual, _module.gelu

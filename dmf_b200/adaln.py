@@ -19,7 +19,7 @@ stream; shift / scale / gate are bf16 or fp32.  ``ln_modulate`` writes its resul
 autocast dtype when autocast is on - the cast autocast would insert before the next Linear.
 Arithmetic is fp32 with one rounding of each result (the reference rounds after every op).
 
-There is no other implementation behind these functions: without the CUDA library they raise.
+There is no other implementation behind ``ln_modulate`` and ``gate_residual``: without the CUDA library they raise.
 """
 
 from __future__ import annotations
@@ -292,3 +292,14 @@ def gate_residual(x: torch.Tensor, gate: torch.Tensor, h: torch.Tensor) -> torch
         return GateResidualFunc.apply(x, None, h, None, gate, None)[0]
     out, tout = GateResidualFunc.apply(xp, xt, hp, ht, gp, gt)
     return fwAD.make_dual(out, tout)
+
+
+def gelu(x: torch.Tensor) -> torch.Tensor:
+    """GELU in its tanh form (the block's MLP), as one kernel for 16-bit CUDA tensors; a dual tensor in gives a dual tensor
+    out, and backward differentiates the primal output only.  Everything else (other types and devices, transforms the
+    native path does not take) is ``torch.nn.functional.gelu``, the same function."""
+    if not torch.compiler.is_compiling():
+        out = _native.gelu(x)
+        if out is not None:
+            return out
+    return torch.nn.functional.gelu(x, approximate="tanh")

@@ -1,4 +1,4 @@
-// C ABI of the adaLN-Zero elementwise ops (include/dmf_adaln.h): validation and launches.
+// C ABI of the transformer block's elementwise ops (include/dmf_adaln.h): validation and launches.
 #include <cuda_runtime.h>
 
 #include <cstring>
@@ -7,6 +7,7 @@
 #include "adaln.cuh"
 #include "dmf_adaln.h"
 #include "dmf_attn.h"
+#include "gelu.cuh"
 
 namespace {
 
@@ -318,6 +319,30 @@ int run_gate_residual_bwd(const dmf_gate_residual_bwd_args* a) {
   return launched();
 }
 
+template <typename T>
+void gelu_launch(const GeluParams& p, unsigned grid, cudaStream_t stream) {
+  if (p.t == nullptr) gelu_kernel<T, true, false><<<grid, kGeluThreads, 0, stream>>>(p);
+  else if (p.y != nullptr) gelu_kernel<T, true, true><<<grid, kGeluThreads, 0, stream>>>(p);
+  else gelu_kernel<T, false, true><<<grid, kGeluThreads, 0, stream>>>(p);
+}
+
+int run_gelu(const dmf_gelu_args* a) {
+  if (a == nullptr || a->x == nullptr || (a->t == nullptr ? a->y == nullptr : a->ty == nullptr)) return DMF_ATTN_ERR_NULL;
+  if (a->dtype != DMF_ATTN_BF16 && a->dtype != DMF_ATTN_FP16) return DMF_ATTN_ERR_DTYPE;
+  const int64_t blocks = (a->count / 8 + kGeluThreads * kGeluVecs - 1) / (kGeluThreads * kGeluVecs);
+  if (a->count < 1 || blocks > 0x7fffffff) return DMF_ATTN_ERR_SHAPE;
+  for (const void* ptr : {a->x, a->t, static_cast<const void*>(a->y), static_cast<const void*>(a->ty)})
+    if ((reinterpret_cast<uintptr_t>(ptr) & 15u) != 0) return DMF_ATTN_ERR_ALIGN;
+  int sms = 0, st;
+  if ((st = sm_count_of_current_device(&sms)) != DMF_ATTN_OK) return st;
+  const GeluParams p = {a->x, a->t, a->y, a->ty, a->count / 8, static_cast<int>(a->count % 8)};
+  const unsigned grid = static_cast<unsigned>(blocks > 0 ? blocks : 1);
+  cudaStream_t stream = static_cast<cudaStream_t>(a->stream);
+  if (a->dtype == DMF_ATTN_BF16) gelu_launch<__nv_bfloat16>(p, grid, stream);
+  else gelu_launch<__half>(p, grid, stream);
+  return launched();
+}
+
 }  // namespace
 
 #define DMF_API __attribute__((visibility("default")))
@@ -331,5 +356,6 @@ DMF_API size_t dmf_adaln_bwd_workspace_bytes(int32_t batch, int32_t seqlen, int3
 DMF_API int dmf_ln_modulate_bwd(const dmf_ln_modulate_bwd_args* args) { return run_ln_modulate_bwd(args); }
 DMF_API int dmf_gate_residual_fwd(const dmf_gate_residual_args* args) { return run_gate_residual_fwd(args); }
 DMF_API int dmf_gate_residual_bwd(const dmf_gate_residual_bwd_args* args) { return run_gate_residual_bwd(args); }
+DMF_API int dmf_gelu(const dmf_gelu_args* args) { return run_gelu(args); }
 
 }  // extern "C"

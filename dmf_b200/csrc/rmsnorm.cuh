@@ -24,6 +24,7 @@
 #include <stdint.h>
 
 #include "sm100_ptx.cuh"
+#include "vec8.cuh"
 
 namespace dmf {
 
@@ -84,30 +85,6 @@ __device__ __forceinline__ float rms_group_sum(float v, int idx, int lane) {
     for (int d = P / 2; d >= 1; d /= 2) v += __shfl_down_sync(0xffffffffu, v, d);
     return __shfl_sync(0xffffffffu, v, lane - idx);
   }
-}
-
-__device__ __forceinline__ uint4 ld_nc_v4(const void* p) {  // read-once data: no L1 allocation
-  uint4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
-               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
-  return v;
-}
-
-template <typename T>
-__device__ __forceinline__ void rms_unpack8(const uint4& v, float (&f)[8]) {
-  const uint32_t u[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float2 a = unpack2<T>(u[i]);
-    f[2 * i] = a.x;
-    f[2 * i + 1] = a.y;
-  }
-}
-
-template <typename T>
-__device__ __forceinline__ void rms_store8(T* p, const float (&f)[8]) {
-  *reinterpret_cast<uint4*>(p) = make_uint4(Pack2<T>::pack(f[0], f[1]), Pack2<T>::pack(f[2], f[3]),
-                                            Pack2<T>::pack(f[4], f[5]), Pack2<T>::pack(f[6], f[7]));
 }
 
 // the weight as the reference uses it: cast to the tensor's 16-bit type first
@@ -191,8 +168,8 @@ __global__ void __launch_bounds__(kRmsThreads) rmsnorm_fwd_kernel(const RmsParam
     for (int u = 0; u < kRmsUnroll; ++u) {
       // (fp32 pairs - two elements per instruction - were tried here: slower at the same register count)
       float x[8], tx[8];
-      rms_unpack8<T>(xr[u], x);
-      if constexpr (kDual) rms_unpack8<T>(tr_[u], tx);
+      unpack8<T>(xr[u], x);
+      if constexpr (kDual) unpack8<T>(tr_[u], tx);
       float ss = 0.f, dot = 0.f;
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
@@ -204,14 +181,14 @@ __global__ void __launch_bounds__(kRmsThreads) rmsnorm_fwd_kernel(const RmsParam
       float y[8];
 #pragma unroll
       for (int i = 0; i < 8; ++i) y[i] = x[i] * r * w[i];
-      if (on[u]) rms_store8(reinterpret_cast<T*>(p.y) + oy[u], y);
+      if (on[u]) store8(reinterpret_cast<T*>(p.y) + oy[u], y);
       if constexpr (kDual) {
         dot = rms_group_sum<C>(dot, idx, lane);
         const float tr = -r * r * r * dot * inv_d;
         float ty[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) ty[i] = fmaf(tx[i], r, x[i] * tr) * w[i];
-        if (on[u]) rms_store8(reinterpret_cast<T*>(p.ty) + oty[u], ty);
+        if (on[u]) store8(reinterpret_cast<T*>(p.ty) + oty[u], ty);
       }
     }
   }
@@ -262,8 +239,8 @@ __global__ void __launch_bounds__(kRmsThreads) rmsnorm_bwd_kernel(const RmsParam
 #pragma unroll
     for (int u = 0; u < kRmsUnroll; ++u) {
       float x[8], dy[8];
-      rms_unpack8<T>(xr[u], x);
-      rms_unpack8<T>(gr[u], dy);
+      unpack8<T>(xr[u], x);
+      unpack8<T>(gr[u], dy);
       float ss = 0.f, xg = 0.f;
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
@@ -276,13 +253,13 @@ __global__ void __launch_bounds__(kRmsThreads) rmsnorm_bwd_kernel(const RmsParam
       const float r = rsqrtf(ss * inv_d + p.eps);
       const float c = r * r * r * xg * inv_d;
       float dx[8], raw[8];
-      rms_unpack8<T>(gr[u], raw);
+      unpack8<T>(gr[u], raw);
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         dx[i] = fmaf(r, dy[i], -x[i] * c);
         dw[i] = fmaf(raw[i], x[i] * r, dw[i]);  // rows that are off hold zeros
       }
-      if (on[u]) rms_store8(reinterpret_cast<T*>(p.dx) + od[u], dx);
+      if (on[u]) store8(reinterpret_cast<T*>(p.dx) + od[u], dx);
     }
   }
   // this block's share of dw: sum over the rows its warps hold side by side

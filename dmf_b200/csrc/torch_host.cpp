@@ -764,6 +764,93 @@ std::optional<Tensor> gate_residual(const Tensor& x_, const Tensor& gate_, const
   return put_back(y, ty, route);
 }
 
+// ---- GELU ----------------------------------------------------------------------------------------------------------------
+
+// one flat run of elements the kernel reads as 16-byte vectors
+Tensor gelu_flat(const Tensor& t) {
+  const Tensor c = t.contiguous();
+  return reinterpret_cast<uintptr_t>(c.data_ptr()) % 16 == 0 ? c : c.clone();
+}
+
+int gelu_launch(const Tensor& x, const Tensor& t, const Tensor& y, const Tensor& ty) {
+  dmf_gelu_args a = {};
+  a.count = x.numel();
+  a.dtype = attn_dtype(x.scalar_type());
+  a.x = x.data_ptr();
+  if (t.defined()) a.t = t.data_ptr();
+  if (y.defined()) a.y = y.data_ptr();
+  if (ty.defined()) a.ty = ty.data_ptr();
+  a.stream = c10::cuda::getCurrentCUDAStream(x.get_device()).stream();
+  return dmf_gelu(&a);  // not in g_launches, which counts the attention, norm and adaLN kernels
+}
+
+PairOut gelu_forward(const Tensor& x_, const Tensor& tx_) {
+  const c10::cuda::CUDAGuard device_guard(x_.device());
+  const Tensor x = gelu_flat(x_);
+  PairOut r;
+  r.y = at::empty(x.sizes(), x.options());
+  Tensor tx;
+  if (tx_.defined()) {
+    tx = gelu_flat(tx_);
+    r.ty = at::empty(x.sizes(), x.options());
+  }
+  r.status = gelu_launch(x, tx, r.y, r.ty);
+  return r;
+}
+
+struct GeluNode : torch::autograd::Function<GeluNode> {
+  static variable_list forward(AutogradContext* ctx, const Tensor& x, const std::optional<Tensor>& tx) {
+    at::AutoDispatchBelowADInplaceOrView below_autograd;
+    PairOut r = gelu_forward(x, value_of(tx));
+    if (r.status != DMF_ATTN_OK) throw RejectedError();
+    ctx->save_for_backward({x});
+    ctx->set_materialize_grads(false);
+    return r.ty.defined() ? variable_list{r.y, r.ty} : variable_list{r.y};
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    at::AutoDispatchBelowADInplaceOrView below_autograd;
+    const auto s = ctx->get_saved_variables();
+    if (!grads[0].defined()) return {at::zeros_like(s[0]), Tensor()};
+    const c10::cuda::CUDAGuard device_guard(s[0].device());
+    TORCH_CHECK(grads[0].sizes() == s[0].sizes() && grads[0].scalar_type() == s[0].scalar_type() &&
+                    grads[0].device() == s[0].device(),
+                "dmf_b200 GELU backward: unexpected gradient");
+    const Tensor x = gelu_flat(s[0]), dy = gelu_flat(grads[0]);
+    const Tensor dx = at::empty(x.sizes(), x.options());
+    const int st = gelu_launch(x, dy, Tensor(), dx);
+    TORCH_CHECK(st == DMF_ATTN_OK, "dmf_attn: ", dmf_attn_status_string(st));
+    return {dx, Tensor()};
+  }
+};
+
+std::optional<Tensor> gelu(const Tensor& x_) {
+  const Route route = find_route();
+  Dual x;
+  if (!route.ok || !split(x_, route, &x)) return std::nullopt;
+  if (attn_dtype(x.p.scalar_type()) < 0 || x.p.numel() == 0) return std::nullopt;
+  if (x.t.defined() && (x.t.sizes() != x.p.sizes() || x.t.scalar_type() != x.p.scalar_type() || x.t.device() != x.p.device()))
+    return std::nullopt;
+  std::optional<BelowTransform> guard(std::in_place, route.jvp);
+  Tensor y, ty;
+  if (needs_grad({&x.p})) {
+    try {
+      variable_list out = GeluNode::apply(x.p, maybe(x.t));
+      y = out[0];
+      if (x.t.defined()) ty = out[1];
+    } catch (const RejectedError&) {
+      return std::nullopt;
+    }
+  } else {
+    at::AutoDispatchBelowADInplaceOrView below_autograd;
+    PairOut r = gelu_forward(x.p, x.t);
+    if (r.status != DMF_ATTN_OK) return std::nullopt;
+    y = r.y;
+    ty = r.ty;
+  }
+  guard.reset();
+  return put_back(y, ty, route);
+}
+
 }  // namespace
 
 PYBIND11_MODULE(_dmf_torch, m) {
@@ -773,6 +860,7 @@ PYBIND11_MODULE(_dmf_torch, m) {
   m.def("rms_norm", &rms_norm, release());
   m.def("ln_modulate", &ln_modulate, release());
   m.def("gate_residual", &gate_residual, release());
+  m.def("gelu", &gelu, release());
   m.def("set_status_word", [](int64_t device, int64_t ptr) {
     TORCH_CHECK(device >= 0 && device < kMaxDevices, "device index out of range");
     g_status_word[device].store(reinterpret_cast<int32_t*>(ptr), std::memory_order_release);

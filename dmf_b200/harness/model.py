@@ -131,11 +131,18 @@ class Attention(nn.Module):
         return self.proj(self.attn(q, k, v).reshape(B, L, C))
 
 
+class FusedGELU(nn.GELU):
+    """nn.GELU(approximate="tanh") through dmf_b200.adaln.gelu: one kernel, tangent included under forward-mode AD."""
+
+    def forward(self, x):
+        return adaln.gelu(x)
+
+
 class Mlp(nn.Module):
-    def __init__(self, in_features: int, hidden_features: int):
+    def __init__(self, in_features: int, hidden_features: int, fused: bool = False):
         super().__init__()
         self.fc1 = nn.Linear(in_features, hidden_features)
-        self.act = nn.GELU(approximate="tanh")
+        self.act = (FusedGELU if fused else nn.GELU)(approximate="tanh")
         self.fc2 = nn.Linear(hidden_features, in_features)
 
     def forward(self, x):
@@ -156,9 +163,9 @@ class DiTBlock(nn.Module):
                               qk_norm=block_kwargs.get("qk_norm", False),
                               attn_func=block_kwargs.get("attn_func", "base"))
         self.norm2 = nn.LayerNorm(hidden_size, elementwise_affine=False, eps=1e-6)
-        self.mlp = Mlp(hidden_size, int(hidden_size * mlp_ratio))
-        self.adaLN_modulation = nn.Sequential(nn.SiLU(), nn.Linear(hidden_size, 6 * hidden_size))
         self.fused = block_kwargs.get("attn_func", "base") in ("fa2", "fa3")   # the B200 ops travel together
+        self.mlp = Mlp(hidden_size, int(hidden_size * mlp_ratio), fused=self.fused)
+        self.adaLN_modulation = nn.Sequential(nn.SiLU(), nn.Linear(hidden_size, 6 * hidden_size))
 
     def forward(self, x, c):
         sh_a, sc_a, g_a, sh_m, sc_m, g_m = self.adaLN_modulation(c).chunk(6, dim=-1)

@@ -143,6 +143,28 @@ typedef struct dmf_gate_residual_bwd_args {
 
 int dmf_gate_residual_bwd(const dmf_gate_residual_bwd_args* args);
 
+/*
+ * GELU in its tanh form, gelu(x) = 0.5 x (1 + tanh(sqrt(2 / pi) (x + 0.044715 x^3))), of the block's MLP
+ * (models/layers.py, DiTBlock: approximate="tanh"), with its tangent, and its primal backward:
+ *   y given, t NULL:   y = gelu(x)
+ *   y and t given:     y = gelu(x), ty = gelu'(x) t
+ *   y NULL, t given:   ty = gelu'(x) t            (the backward: t = dy, ty = dx)
+ * x, t, y, ty: `count` contiguous elements of one 16-bit type, 16-byte aligned; ty is written when t is given, and
+ * y / ty may be x / t themselves.  Arithmetic is fp32 with one rounding of each result.
+ */
+typedef struct dmf_gelu_args {
+  int64_t count;
+  int32_t dtype;                /* enum dmf_attn_dtype (dmf_attn.h): bf16 or fp16 */
+  int32_t reserved;
+  const void* x;
+  const void* t;
+  void* y;
+  void* ty;
+  void* stream;                 /* cudaStream_t */
+} dmf_gelu_args;
+
+int dmf_gelu(const dmf_gelu_args* args);
+
 #ifdef __cplusplus
 }
 #endif
