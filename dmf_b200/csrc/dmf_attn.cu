@@ -837,7 +837,9 @@ int kernel_name(int op, int seqlen_q, int seqlen_kv, int head_dim, int dtype, ch
 
 constexpr int kRmsMaxBlocks = 2048;  // upper bound of the grid, fixes the size of the backward's workspace
 
-int rms_check(int batch, int seqlen, int heads, int d, int dtype) {
+int rms_check(int batch, int seqlen, int heads, int d, int dtype, const void* weight) {
+  if ((dtype & DMF_RMSNORM_WEIGHT_16BIT) != 0 && (reinterpret_cast<uintptr_t>(weight) & 15u) != 0) return DMF_ATTN_ERR_ALIGN;
+  dtype &= ~DMF_RMSNORM_WEIGHT_16BIT;
   if (dtype != DMF_ATTN_BF16 && dtype != DMF_ATTN_FP16) return DMF_ATTN_ERR_DTYPE;
   if (d < 8 || d > 128 || (d % 8) != 0) return DMF_ATTN_ERR_HEAD_DIM;
   if (batch < 1 || heads < 1 || seqlen < 1) return DMF_ATTN_ERR_SHAPE;
@@ -845,10 +847,11 @@ int rms_check(int batch, int seqlen, int heads, int d, int dtype) {
   return DMF_ATTN_OK;
 }
 
-int rms_grid(int64_t rows, int head_dim, int unroll, int sm_count) {
+// one wave of the blocks that are resident at a time
+int rms_grid(int64_t rows, int head_dim, int unroll, int blocks_per_sm, int sm_count) {
   const int64_t block_rows = rms_rows_per_block(head_dim / 8, unroll);
   const int64_t want = (rows + block_rows - 1) / block_rows;
-  int64_t cap = static_cast<int64_t>(sm_count) * 8;  // 8 blocks of 256 threads per SM
+  int64_t cap = static_cast<int64_t>(sm_count) * blocks_per_sm;
   if (cap > kRmsMaxBlocks) cap = kRmsMaxBlocks;
   return static_cast<int>(want < cap ? want : cap);
 }
@@ -881,7 +884,7 @@ bool rms_small(const dmf_attn_tensor& t, int batch, int seqlen, int heads, int d
 
 int run_rmsnorm_fwd(const dmf_rmsnorm_args* a) {
   if (a == nullptr || a->weight == nullptr) return DMF_ATTN_ERR_NULL;
-  int st = rms_check(a->batch, a->seqlen, a->heads, a->head_dim, a->dtype);
+  int st = rms_check(a->batch, a->seqlen, a->heads, a->head_dim, a->dtype, a->weight);
   if (st != DMF_ATTN_OK) return st;
   const bool dual = a->tx.ptr != nullptr;
   if ((st = check_tensor(a->x, 2)) != DMF_ATTN_OK || (st = check_tensor(a->y, 2)) != DMF_ATTN_OK) return st;
@@ -897,16 +900,17 @@ int run_rmsnorm_fwd(const dmf_rmsnorm_args* a) {
     p.ty = a->ty.ptr; p.ty_sb = a->ty.stride_b; p.ty_sl = a->ty.stride_l; p.ty_sh = a->ty.stride_h;
   }
   p.w = a->weight;
+  p.w16 = (a->dtype & DMF_RMSNORM_WEIGHT_16BIT) != 0;
   p.batch = a->batch; p.seqlen = a->seqlen; p.heads = a->heads; p.head_dim = a->head_dim;
   p.rows = static_cast<int64_t>(a->batch) * a->seqlen * a->heads;
   p.eps = a->eps;
-  const int grid = rms_grid(p.rows, a->head_dim, rms_unroll_fwd(dual), sm_count);
+  const int grid = rms_grid(p.rows, a->head_dim, rms_unroll_fwd(dual), kRmsBlocksFwd, sm_count);
   cudaStream_t stream = static_cast<cudaStream_t>(a->stream);
   bool small = true;
   for (const dmf_attn_tensor* t : {&a->x, &a->tx, &a->y, &a->ty})
     small = small && rms_small(*t, a->batch, a->seqlen, a->heads, a->head_dim);
   const int chunks = a->head_dim / 8;
-  if (a->dtype == DMF_ATTN_BF16) {
+  if ((a->dtype & ~DMF_RMSNORM_WEIGHT_16BIT) == DMF_ATTN_BF16) {
     if (small) rms_launch_fwd<__nv_bfloat16, int32_t>(chunks, dual, grid, stream, p);
     else rms_launch_fwd<__nv_bfloat16, int64_t>(chunks, dual, grid, stream, p);
   } else {
@@ -923,7 +927,7 @@ size_t rmsnorm_bwd_workspace_bytes(int d) {
 
 int run_rmsnorm_bwd(const dmf_rmsnorm_bwd_args* a) {
   if (a == nullptr || a->weight == nullptr || a->dweight == nullptr) return DMF_ATTN_ERR_NULL;
-  int st = rms_check(a->batch, a->seqlen, a->heads, a->head_dim, a->dtype);
+  int st = rms_check(a->batch, a->seqlen, a->heads, a->head_dim, a->dtype, a->weight);
   if (st != DMF_ATTN_OK) return st;
   if ((st = check_tensor(a->dy, 2)) != DMF_ATTN_OK || (st = check_tensor(a->x, 2)) != DMF_ATTN_OK ||
       (st = check_tensor(a->dx, 2)) != DMF_ATTN_OK)
@@ -939,17 +943,18 @@ int run_rmsnorm_bwd(const dmf_rmsnorm_bwd_args* a) {
   p.dy = a->dy.ptr; p.dy_sb = a->dy.stride_b; p.dy_sl = a->dy.stride_l; p.dy_sh = a->dy.stride_h;
   p.dx = a->dx.ptr; p.dx_sb = a->dx.stride_b; p.dx_sl = a->dx.stride_l; p.dx_sh = a->dx.stride_h;
   p.w = a->weight;
+  p.w16 = (a->dtype & DMF_RMSNORM_WEIGHT_16BIT) != 0;
   p.dw_partial = static_cast<float*>(a->workspace);
   p.batch = a->batch; p.seqlen = a->seqlen; p.heads = a->heads; p.head_dim = a->head_dim;
   p.rows = static_cast<int64_t>(a->batch) * a->seqlen * a->heads;
   p.eps = a->eps;
-  const int grid = rms_grid(p.rows, a->head_dim, kRmsUnrollBwd, sm_count);
+  const int grid = rms_grid(p.rows, a->head_dim, kRmsUnrollBwd, kRmsBlocksBwd, sm_count);
   cudaStream_t stream = static_cast<cudaStream_t>(a->stream);
   bool small = true;
   for (const dmf_attn_tensor* t : {&a->dy, &a->x, &a->dx})
     small = small && rms_small(*t, a->batch, a->seqlen, a->heads, a->head_dim);
   const int chunks = a->head_dim / 8;
-  if (a->dtype == DMF_ATTN_BF16) {
+  if ((a->dtype & ~DMF_RMSNORM_WEIGHT_16BIT) == DMF_ATTN_BF16) {
     if (small) rms_launch_bwd<__nv_bfloat16, int32_t>(chunks, grid, stream, p);
     else rms_launch_bwd<__nv_bfloat16, int64_t>(chunks, grid, stream, p);
   } else {

@@ -32,7 +32,7 @@ struct RmsParams {
   const void* x;
   const void* tx;     // nullptr: no tangent
   const void* dy;     // backward only
-  const float* w;     // (D) fp32
+  const void* w;      // (D) fp32, or the tensors' 16-bit type when w16
   void* y;
   void* ty;
   void* dx;           // backward only
@@ -46,6 +46,7 @@ struct RmsParams {
   int batch, seqlen, heads, head_dim;
   int64_t rows;
   float eps;
+  int w16;
 };
 
 constexpr int kRmsThreads = 256;
@@ -63,6 +64,12 @@ constexpr int kRmsWarps = kRmsThreads / 32;
 #endif
 __host__ __device__ constexpr int rms_unroll_fwd(bool dual) { return dual ? DMF_RMS_UNROLL_DUAL : DMF_RMS_UNROLL_PLAIN; }
 constexpr int kRmsUnrollBwd = DMF_RMS_UNROLL_BWD;
+// Resident blocks per SM; the grid is one wave of them.  With a grid of 8 blocks per SM the backward ran two full waves and
+// one of a third: 32 x 1024 x 16 rows of 72, L2 flushed, 59.3 -> 54.9 us; forward with tangent 60.4 -> 59.7, without
+// 34.9 -> 33.8.  More blocks with fewer registers each spill (5 blocks forward 72 us, 4 blocks backward 56.8); the next rows'
+// loads issued before the present rows' arithmetic, or three chunks per lane (two shuffles per row sum instead of five),
+// take registers for which a block less is resident: 72 to 80 us and 62 to 66 us forward, 70 and 64 us backward.
+constexpr int kRmsBlocksFwd = 4, kRmsBlocksBwd = 3;
 // A row of C 16-byte chunks takes C neighbouring lanes; a warp holds 32 / C whole rows.
 __host__ __device__ constexpr int rms_rows_per_warp(int chunks) { return 32 / chunks; }
 __host__ __device__ constexpr int rms_rows_per_block(int chunks, int unroll) {
@@ -122,9 +129,20 @@ struct RmsPos {
   }
 };
 
+// the 8 weights of a lane's chunk
+template <typename T>
+__device__ __forceinline__ void rms_weights(const RmsParams& p, int col, float (&w)[8]) {
+  if (p.w16) {
+    unpack8<T>(*reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(p.w) + col), w);
+  } else {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) w[i] = rms_round<T>(reinterpret_cast<const float*>(p.w)[col + i]);
+  }
+}
+
 // head_dim = 8 * C.  Grid-stride over slices of rms_rows_per_block(C) rows.
 template <typename T, int C, bool kDual, typename Off>
-__global__ void __launch_bounds__(kRmsThreads) rmsnorm_fwd_kernel(const RmsParams p) {
+__global__ void __launch_bounds__(kRmsThreads, kRmsBlocksFwd) rmsnorm_fwd_kernel(const RmsParams p) {
   constexpr int R = rms_rows_per_warp(C);
   constexpr int kSlice = R * kRmsWarps;  // rows of one unroll step of the block
   constexpr int kRmsUnroll = rms_unroll_fwd(kDual);
@@ -133,8 +151,7 @@ __global__ void __launch_bounds__(kRmsThreads) rmsnorm_fwd_kernel(const RmsParam
   const int col = idx * 8;
   const bool active = grp < R;
   float w[8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) w[i] = rms_round<T>(p.w[col + i]);
+  rms_weights<T>(p, col, w);
   const float inv_d = 1.f / static_cast<float>(8 * C);
   const uint32_t seqlen = p.seqlen, heads = p.heads;
   const int64_t rows = p.rows;
@@ -195,7 +212,7 @@ __global__ void __launch_bounds__(kRmsThreads) rmsnorm_fwd_kernel(const RmsParam
 }
 
 template <typename T, int C, typename Off>
-__global__ void __launch_bounds__(kRmsThreads) rmsnorm_bwd_kernel(const RmsParams p) {
+__global__ void __launch_bounds__(kRmsThreads, kRmsBlocksBwd) rmsnorm_bwd_kernel(const RmsParams p) {
   constexpr int R = rms_rows_per_warp(C);
   constexpr int kSlice = R * kRmsWarps;
   constexpr int kRmsUnroll = kRmsUnrollBwd;
@@ -205,11 +222,9 @@ __global__ void __launch_bounds__(kRmsThreads) rmsnorm_bwd_kernel(const RmsParam
   const int col = idx * 8;
   const bool active = grp < R;
   float w[8], dw[8];
+  rms_weights<T>(p, col, w);
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    w[i] = rms_round<T>(p.w[col + i]);
-    dw[i] = 0.f;
-  }
+  for (int i = 0; i < 8; ++i) dw[i] = 0.f;
   const float inv_d = 1.f / static_cast<float>(8 * C);
   const uint32_t seqlen = p.seqlen, heads = p.heads;
   const int64_t rows = p.rows;

@@ -404,10 +404,18 @@ std::optional<Tensor> attn_qkvpacked(const Tensor& qkv_, std::optional<double> s
 
 // ---- per-head RMS norm -----------------------------------------------------------------------------------------------
 
+// the weight as the kernel reads it: in the tensors' own 16-bit type where it is there already, else fp32
 Tensor rms_weight(const Tensor& w, const Tensor& x) {
   const Tensor d = w.detach();
+  if (d.scalar_type() == x.scalar_type() && d.device() == x.device() && d.is_contiguous() &&
+      reinterpret_cast<uintptr_t>(d.data_ptr()) % 16 == 0)
+    return d;
   if (d.scalar_type() == at::kFloat && d.device() == x.device() && d.is_contiguous()) return d;
   return d.to(x.options().dtype(at::kFloat)).contiguous();
+}
+
+int rms_dtype(const Tensor& x, const Tensor& w) {
+  return attn_dtype(x.scalar_type()) + (w.scalar_type() == at::kFloat ? 0 : DMF_RMSNORM_WEIGHT_16BIT);
 }
 
 struct PairOut {
@@ -422,7 +430,7 @@ PairOut rms_forward(const Tensor& x_, const Tensor& tx_, const Tensor& weight, d
   r.y = at::empty(x.sizes(), x.options());
   dmf_rmsnorm_args a = {};
   a.batch = x.size(0); a.seqlen = x.size(1); a.heads = x.size(2); a.head_dim = x.size(3);
-  a.dtype = attn_dtype(x.scalar_type());
+  a.dtype = rms_dtype(x, w);
   a.eps = static_cast<float>(eps);
   a.x = t4(x); a.y = t4(r.y);
   Tensor tx;
@@ -431,7 +439,7 @@ PairOut rms_forward(const Tensor& x_, const Tensor& tx_, const Tensor& weight, d
     r.ty = at::empty(x.sizes(), x.options());
     a.tx = t4(tx); a.ty = t4(r.ty);
   }
-  a.weight = w.data_ptr<float>();
+  a.weight = w.data_ptr();
   a.stream = c10::cuda::getCurrentCUDAStream(x.get_device()).stream();
   r.status = w.numel() == x.size(3) ? dmf_rmsnorm_fwd(&a) : static_cast<int>(DMF_ATTN_ERR_SHAPE);
   if (r.status == DMF_ATTN_OK) g_launches.fetch_add(1, std::memory_order_relaxed);
@@ -463,10 +471,10 @@ struct RmsNode : torch::autograd::Function<RmsNode> {
     const Tensor ws = at::empty({static_cast<int64_t>(bytes)}, x.options().dtype(at::kByte));
     dmf_rmsnorm_bwd_args a = {};
     a.batch = x.size(0); a.seqlen = x.size(1); a.heads = x.size(2); a.head_dim = D;
-    a.dtype = attn_dtype(x.scalar_type());
+    a.dtype = rms_dtype(x, w);
     a.eps = static_cast<float>(ctx->saved_data["eps"].toDouble());
     a.dy = t4(dy); a.x = t4(x); a.dx = t4(dx);
-    a.weight = w.data_ptr<float>();
+    a.weight = w.data_ptr();
     a.dweight = dw.data_ptr<float>();
     a.workspace = ws.data_ptr();
     a.workspace_bytes = bytes;

@@ -236,19 +236,22 @@ int dmf_attn_validate_bwd(const dmf_attn_bwd_args* args);
  *   r = rsqrt(mean_d(x^2) + eps)    y = x r w    ty = (tx r - x r^3 mean_d(x tx)) w
  * x, tx, y, ty: (B, L, H, D) tensors in the layout rules above (tx.ptr == NULL: no tangent, ty is
  * not written); weight: D floats in device memory (the module's parameter; it is rounded to the
- * tensors' 16-bit type before use, as the reference casts it).  head_dim: a multiple of 8, at most
+ * tensors' 16-bit type before use, as the reference casts it), or, with DMF_RMSNORM_WEIGHT_16BIT added
+ * to dtype, D elements of that 16-bit type, 16-byte aligned.  head_dim: a multiple of 8, at most
  * 128; seqlen: any positive value.  Arithmetic is fp32 with one rounding of the result.
  */
+#define DMF_RMSNORM_WEIGHT_16BIT 0x100
+
 typedef struct dmf_rmsnorm_args {
   int32_t batch;
   int32_t seqlen;
   int32_t heads;
   int32_t head_dim;
-  int32_t dtype;          /* enum dmf_attn_dtype */
+  int32_t dtype;          /* enum dmf_attn_dtype [+ DMF_RMSNORM_WEIGHT_16BIT] */
   float eps;              /* the reference uses 1e-6 */
   dmf_attn_tensor x, tx;  /* read only */
   dmf_attn_tensor y, ty;  /* out */
-  const float* weight;    /* (D) */
+  const void* weight;     /* (D) fp32, or 16-bit (see above) */
   void* stream;           /* cudaStream_t */
 } dmf_rmsnorm_args;
 
@@ -270,7 +273,7 @@ typedef struct dmf_rmsnorm_bwd_args {
   float eps;
   dmf_attn_tensor dy, x;  /* read only */
   dmf_attn_tensor dx;     /* out */
-  const float* weight;    /* (D) */
+  const void* weight;     /* (D) as for dmf_rmsnorm_fwd */
   float* dweight;         /* out, (D) */
   void* workspace;
   size_t workspace_bytes;

@@ -142,3 +142,21 @@ def test_rejects_bad_arguments():
         ops.rmsnorm_fwd_raw(x, tx, w, 1e-6)                       # CPU tensors: no CPU path
     with pytest.raises(Exception):
         ops.rmsnorm_fwd_raw(x[..., :68].to(DEV), None, w[:68].to(DEV), 1e-6)   # head_dim not a multiple of 8
+
+
+@pytest.mark.parametrize("D", [8, 64, 72, 128])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_weight_in_the_tensors_own_type(D, dtype):
+    """A 16-bit weight is read as it is; an fp32 weight is rounded to that type first, so both give the same bits."""
+    from dmf_b200.rms_norm import rms_norm
+    g = torch.Generator(device=DEV).manual_seed(D)
+    x, tx, dy = (torch.randn(3, 37, 5, D, device=DEV, generator=g).to(dtype) for _ in range(3))
+    w16 = (1 + 0.1 * torch.randn(D + 1, device=DEV, generator=g)).to(dtype)
+    for w in (w16[:D], w16[1:]):                                # the second one is not on a 16-byte boundary
+        outs = []
+        for weight in (w, w.float()):
+            xr, wr = x.clone().requires_grad_(True), weight.detach().requires_grad_(True)
+            y, ty = torch.func.jvp(lambda t: rms_norm(t, wr), (xr,), (tx,))
+            y.backward(dy)
+            outs.append((y, ty, xr.grad, wr.grad.to(dtype)))
+        assert all(torch.equal(a, b) for a, b in zip(*outs))
