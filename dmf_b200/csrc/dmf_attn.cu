@@ -539,30 +539,47 @@ bool bwd_stream_applies(int tail, int seqlen_q, int seqlen_kv) {
   return tail >= 0 && tail <= 16 && !bwd_uses_fused(tail, seqlen_q, seqlen_kv) && bwd_stream_enabled();
 }
 
+size_t delta_smem_bytes(int lrows, int heads) { return static_cast<size_t>(heads) * delta_stride(lrows) * sizeof(float); }
+
+// The two kernels around the main one are compiled per head_dim / 8 = 8..10 (the range of the main kernel).
+template <typename T, int C = 10>
+bool launch_bwd_delta(const BwdStreamParams& p, const dmf_attn_bwd_args* a, cudaStream_t stream) {
+  if constexpr (C > 8) {
+    if (p.head_dim != 8 * C) return launch_bwd_delta<T, C - 1>(p, a, stream);
+  }
+  // positions of a block: kDeltaRows, fewer when the sums of all heads do not fit 48 KB of shared memory
+  int lrows = kDeltaRows;
+  while (lrows > 1 && delta_smem_bytes(lrows, p.heads) > 48 * 1024) lrows /= 2;
+  const size_t smem = delta_smem_bytes(lrows, p.heads);
+  const int64_t blocks = static_cast<int64_t>(p.batch) * (p.seqlen_q / lrows);
+  if (smem > 48 * 1024 || blocks > 0x7fffffff) return false;
+  bwd_delta_kernel<T, C><<<static_cast<unsigned>(blocks), kDeltaThreads, smem, stream>>>(
+      static_cast<const T*>(a->o.ptr), static_cast<const T*>(a->dout.ptr), a->lse, const_cast<float*>(p.ndelta),
+      const_cast<float*>(p.nlse2), p.seqlen_q, p.heads, lrows, a->o.stride_b, a->o.stride_l, a->o.stride_h,
+      a->dout.stride_b, a->dout.stride_l, a->dout.stride_h);
+  return true;
+}
+
+template <typename T, int C = 10>
+void launch_bwd_dq_convert(const BwdStreamParams& p, const dmf_attn_bwd_args* a, cudaStream_t stream) {
+  if constexpr (C > 8) {
+    if (p.head_dim != 8 * C) return launch_bwd_dq_convert<T, C - 1>(p, a, stream);
+  }
+  static_assert(DqConvert<C>::kSmemBytes <= 48 * 1024, "no opt-in needed");
+  bwd_dq_convert_kernel<T, C><<<p.batch * p.heads * p.steps, 256, DqConvert<C>::kSmemBytes, stream>>>(
+      p.dq_acc, static_cast<T*>(a->dq.ptr), p.heads, p.steps, a->dq.stride_b, a->dq.stride_l, a->dq.stride_h, p.scale);
+}
+
 template <typename T, int TAIL>
 int launch_bwd_stream_inst(const BwdStreamParams& p, const dmf_attn_bwd_args* a, int sm_count, cudaStream_t stream) {
   using TR = BwdStreamTraits<TAIL>;
   auto kernel = attn_bwd_stream_kernel<T, TAIL>;
-  auto convert = bwd_dq_convert_kernel<T>;
-  const int convert_smem = (p.head_dim / 4) * 128 * 16;
-  static bool done[64], convert_done[64];
-  if (!allow_smem(kernel, TR::kSmemBytes, done) || !allow_smem(convert, 32 * 128 * 16, convert_done)) return DMF_ATTN_ERR_LAUNCH;
-  // rows of the pre-kernel's block: 32 positions of all heads, fewer when that does not fit 48 KB of shared memory
-  int lrows = 32;
-  while (lrows > 1 && static_cast<size_t>(lrows) * p.heads * (p.head_dim / 8) * sizeof(float) > 48 * 1024) lrows /= 2;
-  const size_t delta_smem = static_cast<size_t>(lrows) * p.heads * (p.head_dim / 8) * sizeof(float);
-  if (delta_smem > 48 * 1024) return DMF_ATTN_ERR_SHAPE;
-  const int64_t want = static_cast<int64_t>(p.batch) * (p.seqlen_q / lrows);
-  const int delta_grid = static_cast<int>(want < 16 * sm_count ? want : 16 * sm_count);
-  bwd_delta_kernel<T><<<delta_grid, 256, delta_smem, stream>>>(
-      static_cast<const T*>(a->o.ptr), static_cast<const T*>(a->dout.ptr), a->lse, const_cast<float*>(p.ndelta),
-      const_cast<float*>(p.nlse2), p.batch, p.seqlen_q, p.heads, p.head_dim, lrows, a->o.stride_b, a->o.stride_l,
-      a->o.stride_h, a->dout.stride_b, a->dout.stride_l, a->dout.stride_h);
+  static bool done[64];
+  if (!allow_smem(kernel, TR::kSmemBytes, done)) return DMF_ATTN_ERR_LAUNCH;
+  if (!launch_bwd_delta<T>(p, a, stream)) return DMF_ATTN_ERR_SHAPE;
   const int grid = p.num_tiles < sm_count ? p.num_tiles : sm_count;
   kernel<<<grid, kBwdStreamThreads, TR::kSmemBytes, stream>>>(p);
-  convert<<<p.batch * p.heads * p.steps, 256, convert_smem, stream>>>(
-      p.dq_acc, static_cast<T*>(a->dq.ptr), p.heads, p.head_dim, p.steps, a->dq.stride_b, a->dq.stride_l,
-      a->dq.stride_h, p.scale);
+  launch_bwd_dq_convert<T>(p, a, stream);
   return cudaGetLastError() == cudaSuccess ? DMF_ATTN_OK : DMF_ATTN_ERR_LAUNCH;
 }
 

@@ -192,3 +192,11 @@ def test_backward_rejects_small_workspace():
     a.lse = lse.data_ptr()
     a.workspace, a.workspace_bytes = None, 0
     assert _lib.load().dmf_attn_bwd(C.byref(a)) == 11
+
+
+@pytest.mark.parametrize("D", [64, 72, 80])
+def test_long_sequence_backward_head_dims(D):
+    """The kernels before and after the main one are compiled per head_dim / 8; five heads leave their last rows ragged."""
+    q, k, v, _, _, _, dout = (x.bfloat16() for x in orc.make_inputs(1, 384, 5, D, seed=D, n_extra=1))
+    _, _, dq, dk, dv = _fwd_bwd((q, k, v), dout)
+    _check((dq, dk, dv), orc.attn_bwd_closed_form(q.float(), k.float(), v.float(), dout.float()))
