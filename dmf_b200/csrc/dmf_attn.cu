@@ -267,10 +267,21 @@ bool fwd_uses_pair(bool dual, int tail, int seqlen_q) {
   return dual && tail >= 0 && tail <= 32 && ((seqlen_q / kBlockQ) % 2 == 0) && pair_kernel_enabled();
 }
 
-// The plain forward takes two query tiles per CTA wherever a head has two.  With one (128 query rows) half of that kernel
-// would idle: the single-CTA kernel, whose two warpgroups share a tile, does 512 x 16 heads x 128 tokens in 124 us
-// instead of 164.
-bool fwd_uses_duo(bool dual, int seqlen_q) { return !dual && seqlen_q >= 2 * kBlockQ; }
+// The plain forward takes two query tiles per CTA (attn_fwd_duo_kernel) or one (attn_fwd_kernel, whose two warpgroups share
+// it).  Two: head_dim <= 96 with an even number of tiles, where o is then the o of the dual pass bit for bit.  Elsewhere by
+// the number of rounds the CTAs take: a round of two tiles costs 1.5 rounds of one at head_dim <= 96 and 1.7 above (1.85 at
+// up to four tiles), so one tile wins where its rounds are fewer than that, and always in a single round.  us, two tiles
+// against one, in brackets the rounds of one / of two: head_dim 72, 9 tiles, 16 heads (1/1) 18.0 / 15.3, 64 (4/3) 50.1 / 46.3,
+// 96 (6/4) 65.0 / 66.2, 256 (16/9) 138 / 171; head_dim 128, 3 tiles, 640 heads (13/9) 81.6 / 64.8; 5 tiles, 256 heads (9/6)
+// 73.3 / 65.9; 9 tiles, 64 heads (4/3) 57.0 / 48.6, 200 (13/7) 135 / 146; 16 tiles, 48 heads (6/3) 96 / 114.
+bool fwd_uses_duo(bool dual, int head_dim, int64_t batch_heads, int q_tiles, int sm_count) {
+  if (dual || q_tiles < 2) return false;
+  if (head_dim <= 96 && q_tiles % 2 == 0) return true;
+  const int64_t one = (batch_heads * q_tiles + sm_count - 1) / sm_count;
+  const int64_t two = (batch_heads * ((q_tiles + 1) / 2) + sm_count - 1) / sm_count;
+  const int cost = head_dim <= 96 ? 150 : q_tiles <= 4 ? 185 : 170;  // a round of two tiles, in hundredths of a round of one
+  return one > 1 && 100 * one >= cost * two;
+}
 
 int run_fwd(const dmf_attn_fwd_args* a, bool dual, bool f32out = false) {
   int st = validate_fwd(a, dual, f32out ? 4 : 2);
@@ -284,7 +295,7 @@ int run_fwd(const dmf_attn_fwd_args* a, bool dual, bool f32out = false) {
   const int B = a->batch, H = a->heads, D = a->head_dim, Lq = a->seqlen_q, Lk = a->seqlen_kv, dt = a->dtype;
   if ((st = make_map_pair(&p.q_main, &p.q_tail, a->q, dt, B, Lq, H, D, tail, kBlockQ)) != DMF_ATTN_OK) return st;
   // CTA-pair kernel: dual pass, P in its own tensor-memory columns (head_dim <= 96), tiles pair up
-  const bool duo = fwd_uses_duo(dual, Lq);
+  const bool duo = fwd_uses_duo(dual, D, static_cast<int64_t>(B) * H, Lq / kBlockQ, sm_count);
   const bool pair = fwd_uses_pair(dual, tail, Lq);
   if (f32out && !(pair && dt == DMF_ATTN_BF16 && tail <= 16)) return DMF_ATTN_ERR_HEAD_DIM;
   const int k_box_rows = pair ? kBlockKV / 2 : kBlockKV;  // a CTA of a pair loads half of the key rows
@@ -832,7 +843,7 @@ int kernel_name(int op, int seqlen_q, int seqlen_kv, int head_dim, int dtype, ch
   const char* t = dtype == DMF_ATTN_BF16 ? "bf16" : "fp16";
   if (op == 0 || op == 1) {
     const char* kind = op == 0 ? "dual" : "plain";
-    if (fwd_uses_duo(op == 0, seqlen_q)) {
+    if (fwd_uses_duo(op == 0, head_dim, 148 * 64, seqlen_q / kBlockQ, 148)) {  // with heads enough to fill the GPU
       std::snprintf(buf, len, "attn_fwd_duo_kernel<%s, TAIL=%d> (two query tiles per CTA)", t, tail);
     } else if (fwd_uses_pair(op == 0, tail, seqlen_q)) {
       const bool is_short = tail == 16 && seqlen_kv <= kShortMaxBlocks * kBlockKV;

@@ -13,8 +13,8 @@ pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
 
 
-@pytest.mark.parametrize("shape", [(1, 256, 128, 1, 64), (2, 384, 256, 3, 72), (40, 384, 128, 8, 72), (12, 640, 640, 7, 64),
-                                   (3, 256, 1152, 5, 80), (30, 384, 384, 4, 96), (24, 384, 256, 5, 128), (1, 2048, 2048, 2, 104)])
+@pytest.mark.parametrize("shape", [(1, 256, 128, 1, 64), (16, 384, 256, 4, 72), (25, 384, 128, 8, 72), (12, 640, 640, 7, 64),
+                                   (3, 256, 1152, 5, 80), (30, 384, 384, 4, 96), (20, 1024, 128, 5, 128), (8, 2048, 512, 6, 104)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_plain_forward_two_tiles_per_cta(shape, dtype):
     B, Lq, Lk, H, D = shape
@@ -29,4 +29,17 @@ def test_plain_forward_two_tiles_per_cta(shape, dtype):
         # P and o are rounded to 8 (11) bits: 2^-9 (2^-12) relative each, independent over the keys
         assert orc.rel_l2(o[b:b + 1].float().cpu(), o_ref) < (6e-3 if dtype == torch.bfloat16 else 1e-3)
         # a quarter of the exponentials are cubics with 7.5e-5 relative error
+        assert float((lse[b:b + 1].cpu().double() - lse_ref).abs().max()) < 1e-4
+
+
+@pytest.mark.parametrize("shape", [(2, 384, 256, 3, 72), (40, 384, 128, 8, 72), (24, 384, 256, 5, 128), (1, 2048, 2048, 2, 104)])
+def test_plain_forward_one_tile_per_cta_where_that_takes_fewer_rounds(shape):
+    """Odd tile counts and head_dim above 96 with few heads: the other kernel, to the same tolerances."""
+    B, Lq, Lk, H, D = shape
+    q = orc.make_inputs(B, Lq, H, D, seed=Lq + D)[0].bfloat16()
+    k, v = (x.bfloat16() for x in orc.make_inputs(B, Lk, H, D, seed=Lk + H)[1:3])
+    o, _, lse, _ = _cabi.fwd(*(x.to(DEV) for x in (q, k, v)))
+    for b in {0, B - 1}:
+        o_ref, lse_ref = orc.attn_fwd_closed_form(*[x[b:b + 1].float() for x in (q, k, v)])
+        assert orc.rel_l2(o[b:b + 1].float().cpu(), o_ref) < 6e-3
         assert float((lse[b:b + 1].cpu().double() - lse_ref).abs().max()) < 1e-4
