@@ -1,14 +1,17 @@
 // GELU (tanh form) of the transformer block's MLP with its tangent, and its primal backward.
 //
-//   s(x) = 1 / (1 + exp(-2 u)),  u = sqrt(2 / pi) (x + 0.044715 x^3)        gelu(x)  = x s
-//                                                                            gelu'(x) = s + 2 x u' s (1 - s)
+//   u(x) = sqrt(2 / pi) (x + 0.044715 x^3),  h = tanh u                     gelu(x)  = 0.5 x (1 + h)
+//                                                                           gelu'(x) = 0.5 (1 + h) + 0.5 x (1 - h^2) u'
 //   y = gelu(x)        ty = gelu'(x) tx        dx = gelu'(x) dy
 //
-// (0.5 (1 + tanh u) = s: the logistic form has no cancellation for negative x and takes one exponential and one reciprocal.)
-// What bounds it: HBM.  The tensors are the widest of the model (4 C per token) and nothing is computed between them.  Each
-// thread has kGeluVecs 16-byte loads of each tensor in flight and ends: a grid-stride loop over 4 to 8 blocks per SM is 10 to
-// 15 % slower.  8192 x 4608 bf16 with L2 flushed (75 MB a tensor), of the measured copy rate: y alone 29 us (0.79), y and ty
-// 53 us (0.87), backward 41 us (0.84); the library's kernels take 39, 39 + 50 and 50 us.
+// The arithmetic is pinned operation by operation (which products are fused into sums): every 16-bit result is the library's
+// bit for bit, so a model gives the same outputs whichever of the two runs, limits and overflows included.  (The logistic
+// form x / (1 + exp(-2 u)) is shorter, 10 us on y alone and 6 us on the backward below, but rounds differently, and its
+// derivative is NaN where x^3 overflows and gelu' is 0 or 1.)
+// What bounds it: HBM, and for y alone tanhf.  The tensors are the widest of the model (4 C per token).  Each thread has
+// kGeluVecs 16-byte loads of each tensor in flight and ends: a grid-stride loop over 4 to 8 blocks per SM is 10 to 15 %
+// slower.  8192 x 4608 bf16 with L2 flushed (75 MB a tensor), of the measured copy rate: y alone 39 us (0.59), y and ty
+// 53 us (0.87), backward 47 us (0.74); the library's kernels take 43, 43 + 53 and 53 us.
 #pragma once
 
 #include <stdint.h>
@@ -29,13 +32,20 @@ struct GeluParams {
 constexpr int kGeluThreads = 256;
 constexpr int kGeluVecs = 4;
 
-__device__ __forceinline__ float gelu_s(float x) {
-  const float z = x * fmaf(x * x, -2.f * 0.7978845608028654f * 0.044715f, -2.f * 0.7978845608028654f);  // -2 u
-  return __fdividef(1.f, 1.f + __expf(z));
+constexpr float kGeluC = 0.7978845608028654f;  // sqrt(2 / pi)
+constexpr float kGeluK = 0.044715f;
+
+// tanh u(x)
+__device__ __forceinline__ float gelu_tanh(float x) {
+  const float cube = __fmul_rn(__fmul_rn(x, x), x);
+  return tanhf(__fmul_rn(kGeluC, fmaf(kGeluK, cube, x)));
 }
-__device__ __forceinline__ float gelu_grad(float x, float s) {
-  const float du2 = fmaf(x * x, 6.f * 0.7978845608028654f * 0.044715f, 2.f * 0.7978845608028654f);  // 2 u'
-  return fmaf(x * du2, s * (1.f - s), s);
+// h = tanh u(x)
+__device__ __forceinline__ float gelu_value(float x, float h) { return __fmul_rn(__fmul_rn(0.5f, x), __fadd_rn(1.f, h)); }
+__device__ __forceinline__ float gelu_grad(float x, float h) {
+  const float du = __fmul_rn(kGeluC, fmaf(3.f * kGeluK, __fmul_rn(x, x), 1.f));
+  const float right = __fmul_rn(__fmul_rn(0.5f, x), fmaf(-h, h, 1.f));
+  return fmaf(right, du, __fmul_rn(0.5f, __fadd_rn(1.f, h)));
 }
 
 // kY: writes gelu(x); kT: writes gelu'(x) t
@@ -61,9 +71,9 @@ __global__ void __launch_bounds__(kGeluThreads) gelu_kernel(const GeluParams p) 
     if constexpr (kT) unpack8<T>(tv[u], b);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      const float s = gelu_s(a[j]);
-      if constexpr (kT) b[j] *= gelu_grad(a[j], s);
-      a[j] *= s;
+      const float h = gelu_tanh(a[j]);
+      if constexpr (kT) b[j] *= gelu_grad(a[j], h);
+      if constexpr (kY) a[j] = gelu_value(a[j], h);
     }
     if constexpr (kY) store8(reinterpret_cast<T*>(p.y) + 8 * i, a);
     if constexpr (kT) store8(reinterpret_cast<T*>(p.ty) + 8 * i, b);
@@ -71,10 +81,10 @@ __global__ void __launch_bounds__(kGeluThreads) gelu_kernel(const GeluParams p) 
   if (blockIdx.x == 0 && threadIdx.x < p.tail) {
     const int64_t i = 8 * p.n8 + threadIdx.x;
     const float a = static_cast<float>(reinterpret_cast<const T*>(p.x)[i]);
-    const float s = gelu_s(a);
+    const float h = gelu_tanh(a);
     float b = 0.f;
-    if constexpr (kT) b = gelu_grad(a, s) * static_cast<float>(reinterpret_cast<const T*>(p.t)[i]);
-    if constexpr (kY) reinterpret_cast<T*>(p.y)[i] = static_cast<T>(a * s);
+    if constexpr (kT) b = gelu_grad(a, h) * static_cast<float>(reinterpret_cast<const T*>(p.t)[i]);
+    if constexpr (kY) reinterpret_cast<T*>(p.y)[i] = static_cast<T>(gelu_value(a, h));
     if constexpr (kT) reinterpret_cast<T*>(p.ty)[i] = static_cast<T>(b);
   }
 }

@@ -55,3 +55,25 @@ def test_limits_strides_and_other_types():
     f = torch.randn(33, device=DEV)
     assert torch.equal(adaln.gelu(f), torch.nn.functional.gelu(f, approximate="tanh"))
     assert adaln.gelu(a[:0]).shape == (0, 48)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_every_value_is_the_library_s_bit_for_bit(dtype):
+    """All 65536 inputs: the value; and the tangent and the gradient for several factors each (NaN where the library's are)."""
+    lib = lambda x: torch.nn.functional.gelu(x, approximate="tanh")
+    same = lambda a, b: bool(((a == b) | (a.isnan() & b.isnan())).all())
+    x = torch.arange(-32768, 32768, dtype=torch.int32, device=DEV).to(torch.int16).view(dtype)
+    assert ops._CHECK_EVERY_CALL or _native.gelu(x) is not None
+    assert same(adaln.gelu(x), lib(x))
+    for seed in range(8):
+        t = torch.randn(65536, device=DEV, generator=torch.Generator(device=DEV).manual_seed(seed)).to(dtype)
+        res = []
+        for fn in (adaln.gelu, lib):
+            xr = x.clone().requires_grad_(True)
+            y, ty = torch.func.jvp(fn, (xr,), (t,))
+            res.append((y, ty, *torch.autograd.grad(y, xr, t)))
+        assert all(same(a, b) for a, b in zip(*res, strict=True))
+    # finite where the function is: x^3 overflows above 7e12, and gelu' is 0 or 1 there
+    big = torch.tensor([2e13, -2e13, 1e18, -1e18], device=DEV).bfloat16().requires_grad_(True)
+    y, ty = torch.func.jvp(adaln.gelu, (big,), (torch.ones_like(big),))
+    assert ty.tolist() == [1, 0, 1, 0] and torch.autograd.grad(y.sum(), big)[0].tolist() == [1, 0, 1, 0]
