@@ -6,13 +6,21 @@
 namespace dmf {
 namespace {
 
-template <typename T, int TAIL>
-int launch(const FwdParams& p, int grid, cudaStream_t stream) {
+template <typename T, int TAIL, bool kCubics>
+int launch_inst(const FwdParams& p, int grid, cudaStream_t stream) {
   static bool done[64];
-  auto kernel = attn_fwd_duo_kernel<T, TAIL>;
+  auto kernel = attn_fwd_duo_kernel<T, TAIL, kCubics>;
   if (!allow_smem(kernel, DuoTraits<TAIL>::kSmemBytes, done)) return DMF_ATTN_ERR_LAUNCH;
   kernel<<<grid, kDuoThreads, DuoTraits<TAIL>::kSmemBytes, stream>>>(p);
   return cudaGetLastError() == cudaSuccess ? DMF_ATTN_OK : DMF_ATTN_ERR_LAUNCH;
+}
+
+template <typename T, int TAIL>
+int launch(const FwdParams& p, int grid, cudaStream_t stream) {
+  if constexpr (duo_cubics(TAIL, 2)) {
+    if (duo_cubics(TAIL, p.num_q_tiles)) return launch_inst<T, TAIL, true>(p, grid, stream);
+  }
+  return launch_inst<T, TAIL, false>(p, grid, stream);
 }
 
 template <typename T>

@@ -9,7 +9,7 @@
 // softmax warps of its own: while one tile waits for its products the other computes.  K and V blocks are shared.
 //
 // Measured (one B200, sustained; the power limit is reached, the SM clock falls to 1.64 GHz): 64 x 16 heads x 1024 tokens,
-// head_dim 72: 549 -> 462 us; 256 x 16 x 256 tokens, 72: 191 -> 166 us; 16 x 12 x 2048 tokens, 128: 460 -> 419 us.
+// head_dim 72: 549 -> 462 us; 256 x 16 x 256 tokens, 72: 191 -> 166 us; 16 x 12 x 2048 tokens, 128: 395 -> 363 us.
 // Within 1 % of it or slower: P in columns of its own (one buffer the tiles take in turn) with S issued a block or two
 // ahead, with one or two MMA-issuing warps (shorter in cycles, at a lower clock; 15 % slower at two blocks per tile); a
 // score row shared by two warps, the maximum exchanged through shared memory (10 % slower).
@@ -26,8 +26,11 @@
 // Query tiles are double-buffered where shared memory allows (head_dim <= 96); the output tile is staged in the query
 // tile's own buffer, which is dead by then, and leaves by TMA store.
 //
-// The per-row arithmetic (order of the sums, lazy maximum, which exponentials are cubics) is that of attn_fwd_pair.cuh:
-// o is bit for bit the primal output of the dual pass.
+// Two variants of the per-row arithmetic, by the shape of one (batch, head) alone (duo_cubics).  With an even number of tiles
+// and head_dim <= 96 it is that of attn_fwd_pair.cuh (order of the sums, a quarter of the exponentials cubics): o is bit for
+// bit the primal output of the dual pass.  Elsewhere it is that of attn_fwd_kernel, which takes these shapes too when they
+// are few (fwd_uses_duo in dmf_attn.cu): all exponentials on the MUFU unit, a row's sum as two halves.  So o and lse of an
+// element never depend on how many others are in the batch.
 #pragma once
 
 #include "attn_fwd.cuh"
@@ -60,9 +63,12 @@ struct DuoTraits {
 
 constexpr int kDuoThreads = 320;
 
+// whether the arithmetic is that of the pair kernel (see above)
+constexpr bool duo_cubics(int tail, int num_q_tiles) { return tail <= 32 && num_q_tiles % 2 == 0; }
+
 // p.num_tiles counts units: p.unit_tiles (1 or 2) neighbouring query tiles of one (batch, head); with an odd number of
 // tiles the last unit of a head has one.
-template <typename T, int TAIL>
+template <typename T, int TAIL, bool kCubics>
 __global__ void __launch_bounds__(kDuoThreads, 1)
 attn_fwd_duo_kernel(const __grid_constant__ FwdParams p) {
   using TR = DuoTraits<TAIL>;
@@ -243,7 +249,7 @@ attn_fwd_duo_kernel(const __grid_constant__ FwdParams p) {
       const int bh = u / units_per_bh, b = bh / p.heads, h = bh % p.heads;
       const int q0 = (p.unit_tiles * (u % units_per_bh) + slot) * kBlockQ;
       const uint32_t buf = qcnt % TR::kQBufs;
-      float m_used = -CUDART_INF_F, l = 0.f;
+      float m_used = -CUDART_INF_F, l = 0.f, l_hi = 0.f;  // l_hi (!kCubics): the sum over key columns 64 to 127
       for (int j = 0; j < num_kv_blocks; ++j, ++scnt) {
         ok = wait(TR::kBarSFull + slot, scnt & 1u);
         if (!ok) break;
@@ -275,6 +281,7 @@ attn_fwd_duo_kernel(const __grid_constant__ FwdParams p) {
               m_used = m_blk;
             }
             l *= alpha;
+            l_hi *= alpha;
 #pragma unroll 1
             for (int c = 0; c < DPAD / 16; ++c) {
               uint32_t a[16];
@@ -296,7 +303,7 @@ attn_fwd_duo_kernel(const __grid_constant__ FwdParams p) {
             float x0, x1, p2, p3;
             unpack_f2(fma2(pack_u2(r[c][i], r[c][i + 1]), sl2_2, neg_m2), x0, x1);
             const uint64_t xb = fma2(pack_u2(r[c][i + 2], r[c][i + 3]), sl2_2, neg_m2);
-            if (kPolyEvery > 0 && ((i / 4) % (kPolyEvery > 0 ? kPolyEvery : 1)) == (kPolyEvery - 1)) {
+            if (kCubics && kPolyEvery > 0 && ((i / 4) % (kPolyEvery > 0 ? kPolyEvery : 1)) == (kPolyEvery - 1)) {
               poly_exp2_x2(xb, p2, p3);
             } else {
               float x2, x3;
@@ -311,11 +318,12 @@ attn_fwd_duo_kernel(const __grid_constant__ FwdParams p) {
             pk[i / 2 + 1] = Pack2<T>::pack(p2, p3);
           }
           tmem_st_x16(t_s + c * 16, pk);  // over S columns this warp holds in registers
-        }
-        {
-          float s0, s1;
-          unpack_f2(add2(la, lb), s0, s1);
-          l += s0 + s1;
+          if (c == 3 || (!kCubics && c == 1)) {
+            float s0, s1;
+            unpack_f2(add2(la, lb), s0, s1);
+            (!kCubics && c == 3 ? l_hi : l) += s0 + s1;
+            la = lb = pack_f2(0.f, 0.f);
+          }
         }
         tmem_wait_st();
         tc_fence_before_sync();
@@ -328,6 +336,7 @@ attn_fwd_duo_kernel(const __grid_constant__ FwdParams p) {
       ok = named_bar_and(1 + slot, 128, ok);  // every warp of the slot arrives here, whatever happened to its waits
       if (!ok) break;
       tc_fence_after_sync();
+      if constexpr (!kCubics) l += l_hi;
       const float inv_l = 1.f / l;
       p.lse[(static_cast<int64_t>(b) * p.heads + h) * p.seqlen_q + q0 + row] =
           (m_used + __log2f(l)) * 0.6931471805599453f;

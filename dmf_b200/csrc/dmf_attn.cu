@@ -268,18 +268,22 @@ bool fwd_uses_pair(bool dual, int tail, int seqlen_q) {
 }
 
 // The plain forward takes two query tiles per CTA (attn_fwd_duo_kernel) or one (attn_fwd_kernel, whose two warpgroups share
-// it).  Two: head_dim <= 96 with an even number of tiles, where o is then the o of the dual pass bit for bit.  Elsewhere by
-// the number of rounds the CTAs take: a round of two tiles costs 1.5 rounds of one at head_dim <= 96 and 1.7 above (1.85 at
-// up to four tiles), so one tile wins where its rounds are fewer than that, and always in a single round.  us, two tiles
-// against one, in brackets the rounds of one / of two: head_dim 72, 9 tiles, 16 heads (1/1) 18.0 / 15.3, 64 (4/3) 50.1 / 46.3,
-// 96 (6/4) 65.0 / 66.2, 256 (16/9) 138 / 171; head_dim 128, 3 tiles, 640 heads (13/9) 81.6 / 64.8; 5 tiles, 256 heads (9/6)
-// 73.3 / 65.9; 9 tiles, 64 heads (4/3) 57.0 / 48.6, 200 (13/7) 135 / 146; 16 tiles, 48 heads (6/3) 96 / 114.
+// it).  Two: head_dim <= 96 with an even number of tiles, where o is then the o of the dual pass bit for bit.  Elsewhere, where
+// both give the same bits, by the number of rounds the CTAs take: one tile wins where its rounds are fewer than those of two
+// times what such a round costs, 1.55 at head_dim <= 96 and 1.7 above (1.9 at up to four tiles: a short tile's start and end
+// are not hidden; with two tiles and more than two rounds the gain is gone), and always in a single round.  us, one tile
+// against two, in brackets the rounds: head_dim 72, 9 tiles, 12 heads (1/1) 15.2 / 18.4, 64 (4/3) 47.8 / 55.6, 96 (6/4)
+// 68.4 / 72.1, 128 (8/5) 91.3 / 85.3, 256 (16/9) 176 / 150; 5 tiles, 200 heads (7/5) 49.6 / 52.8, 400 (14/9) 95.2 / 88.6;
+// head_dim 128, 2 tiles, 128 heads (2/1) 11.8 / 10.1, 400 (6/3) 27.2 / 29.9; 4 tiles, 256 heads (7/4) 47.5 / 49.7, 640 (18/9)
+// 108 / 103; 5 tiles, 256 heads (9/6) 68.4 / 77.0; 9 tiles, 64 heads (4/3) 50.0 / 61.3, 200 (13/7) 150 / 138; 16 tiles,
+// 48 heads (6/3) 118 / 101.
 bool fwd_uses_duo(bool dual, int head_dim, int64_t batch_heads, int q_tiles, int sm_count) {
   if (dual || q_tiles < 2) return false;
   if (head_dim <= 96 && q_tiles % 2 == 0) return true;
   const int64_t one = (batch_heads * q_tiles + sm_count - 1) / sm_count;
   const int64_t two = (batch_heads * ((q_tiles + 1) / 2) + sm_count - 1) / sm_count;
-  const int cost = head_dim <= 96 ? 150 : q_tiles <= 4 ? 185 : 170;  // a round of two tiles, in hundredths of a round of one
+  if (head_dim > 96 && q_tiles == 2 && two > 2) return false;
+  const int cost = head_dim <= 96 ? 155 : q_tiles <= 4 ? 190 : 170;  // a round of two tiles, in hundredths of a round of one
   return one > 1 && 100 * one >= cost * two;
 }
 
@@ -843,7 +847,8 @@ int kernel_name(int op, int seqlen_q, int seqlen_kv, int head_dim, int dtype, ch
   const char* t = dtype == DMF_ATTN_BF16 ? "bf16" : "fp16";
   if (op == 0 || op == 1) {
     const char* kind = op == 0 ? "dual" : "plain";
-    if (fwd_uses_duo(op == 0, head_dim, 148 * 64, seqlen_q / kBlockQ, 148)) {  // with heads enough to fill the GPU
+    const int q_tiles = seqlen_q / kBlockQ, units = (q_tiles + 1) / 2;
+    if (fwd_uses_duo(op == 0, head_dim, units < 148 ? 148 / units : 1, q_tiles, 148)) {  // as many heads as fill the GPU once
       std::snprintf(buf, len, "attn_fwd_duo_kernel<%s, TAIL=%d> (two query tiles per CTA)", t, tail);
     } else if (fwd_uses_pair(op == 0, tail, seqlen_q)) {
       const bool is_short = tail == 16 && seqlen_kv <= kShortMaxBlocks * kBlockKV;

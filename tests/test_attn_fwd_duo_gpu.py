@@ -43,3 +43,19 @@ def test_plain_forward_one_tile_per_cta_where_that_takes_fewer_rounds(shape):
         o_ref, lse_ref = orc.attn_fwd_closed_form(*[x[b:b + 1].float() for x in (q, k, v)])
         assert orc.rel_l2(o[b:b + 1].float().cpu(), o_ref) < 6e-3
         assert float((lse[b:b + 1].cpu().double() - lse_ref).abs().max()) < 1e-4
+
+
+@pytest.mark.parametrize("shape", [(16, 384, 256, 4, 72), (25, 640, 384, 8, 64), (32, 640, 384, 4, 96), (20, 1024, 256, 5, 128),
+                                   (12, 1152, 1152, 12, 128), (64, 512, 512, 4, 72)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_plain_forward_bits_do_not_depend_on_the_batch(shape, dtype):
+    """One element alone takes one tile per CTA, the batch two: the same o and lse bit for bit, late maxima included."""
+    B, Lq, Lk, H, D = shape
+    q = orc.make_inputs(B, Lq, H, D, seed=Lq + D)[0].to(dtype)
+    k, v = (x.to(dtype) for x in orc.make_inputs(B, Lk, H, D, seed=Lk + H)[1:3])
+    k = k * torch.linspace(0.5, 6.0, Lk).view(1, Lk, 1, 1).to(dtype)
+    q, k, v = (x.to(DEV) for x in (q, k, v))
+    o, _, lse, _ = _cabi.fwd(q, k, v)
+    for b in {0, B // 2, B - 1}:
+        o1, _, lse1, _ = _cabi.fwd(*(x[b:b + 1].contiguous() for x in (q, k, v)))
+        assert torch.equal(o[b:b + 1], o1) and torch.equal(lse[b:b + 1], lse1)
