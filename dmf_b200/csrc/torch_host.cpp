@@ -9,8 +9,8 @@
 //   * exactly one functorch JVP level (torch.func.jvp, how loss.py:165-170 reaches the ops): the inputs are unwrapped to
 //     the tensors below that level, the op runs there - autograd at that level as usual - and primal and tangent are
 //     wrapped again;
-//   * anything else (tensor subclasses, dispatch modes, vmap / grad / nested transforms, arguments that the op rejects,
-//     CPU tensors) returns None, and the Python caller takes the general route, which also raises the exact errors.
+//   * anything else (tensor subclasses, dispatch modes, jit tracing, vmap / grad / nested transforms, arguments that the op
+//     rejects, CPU tensors) returns None, and the Python caller takes the general route, which also raises the exact errors.
 //
 // Semantics are those of the autograd.Functions in flash_attn_jvp.py, rms_norm.py and adaln.py: tangents are plain
 // inputs, backward differentiates the primal outputs only, tangent outputs carry no gradient.
@@ -23,6 +23,7 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/custom_function.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 #include <torch/extension.h>
 
 #include <atomic>
@@ -69,6 +70,7 @@ struct Route {
 Route find_route() {
   Route r;
   if (c10::impl::TorchDispatchModeTLS::any_modes_set()) return r;
+  if (torch::jit::tracer::isTracing()) return r;  // a trace has to see an op: a launch from here would leave no node in it
   const auto& stack = ft::getDynamicLayerStack();
   if (stack.empty()) {
     r.ok = true;

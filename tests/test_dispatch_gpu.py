@@ -1,0 +1,50 @@
+"""What a call through torch's dispatcher keeps, whichever host path the op takes: tracing, second derivatives, batched
+gradients, tangents that are differentiated, saved-tensor hooks, tensor subclasses and function modes."""
+
+import pytest
+import torch
+from torch.overrides import TorchFunctionMode
+
+from dmf_b200 import adaln, flash_attn_func, flash_attn_qkvpacked_func
+from dmf_b200.rms_norm import rms_norm
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _randn(*shape, dtype=torch.bfloat16, seed=0):
+    g = torch.Generator(device=DEV).manual_seed(seed + sum(shape))
+    return torch.randn(*shape, device=DEV, dtype=dtype, generator=g)
+
+
+def _case(op, seed=0):
+    """(function, its tensor inputs)"""
+    r = lambda *s, **k: _randn(*s, seed=seed + 1000 * len(made), **k)
+    made = []
+
+    def new(*s, **k):
+        made.append(r(*s, **k))
+        return made[-1]
+
+    if op == "attn":
+        return flash_attn_func, [new(2, 256, 3, 72), new(2, 256, 3, 72), new(2, 256, 3, 72)]
+    if op == "packed":
+        return flash_attn_qkvpacked_func, [new(2, 128, 3, 2, 64)]
+    if op == "rms":
+        return rms_norm, [new(2, 20, 3, 72), new(72, dtype=torch.float32)]
+    if op == "ln":
+        return adaln.ln_modulate, [new(2, 24, 384), new(2, 1, 384), new(2, 1, 384)]
+    if op == "gate":
+        return adaln.gate_residual, [new(2, 24, 384), new(2, 1, 384), new(2, 24, 384)]
+    return adaln.gelu, [new(3, 50, 40)]
+
+
+ALL = ("attn", "packed", "rms", "ln", "gate", "gelu")
+
+
+@pytest.mark.parametrize("op", ALL)
+def test_a_traced_call_replays_on_new_inputs(op):
+    fn, args = _case(op)
+    traced = torch.jit.trace(fn, tuple(args))
+    new = _case(op, seed=7)[1]
+    assert torch.equal(traced(*new), fn(*new))
