@@ -190,6 +190,25 @@ def _like(grad: torch.Tensor, ref_shape, ref_dtype) -> torch.Tensor:
     return grad.to(ref_dtype).reshape(ref_shape)
 
 
+class _FirstOrderOnly(torch.autograd.Function):
+    """The kernels' gradients under create_graph: differentiating them raises instead of leaving a term out."""
+
+    @staticmethod
+    def forward(ctx, n, *tensors):
+        return tuple(t.detach() for t in tensors[:n])
+
+    @staticmethod
+    def backward(ctx, *unused):
+        raise RuntimeError("dmf_b200 ops have no second derivatives")
+
+
+def _first_order_only(grads, *sources):
+    if (not torch.is_grad_enabled() or not any(t.requires_grad for t in sources)
+            or torch._C._functorch.peek_interpreter_stack() is not None):
+        return grads
+    return _FirstOrderOnly.apply(len(grads), *grads, *sources)
+
+
 class LnModulateFunc(torch.autograd.Function):
 
     @staticmethod
@@ -211,7 +230,9 @@ class LnModulateFunc(torch.autograd.Function):
         x, scale = ctx.saved_tensors
         dx, dshift, dscale = ln_modulate_bwd_raw(dy, x, scale, ctx.eps)
         s_shape, s_dtype, c_shape, c_dtype = ctx.mod_meta
-        return dx, None, _like(dshift, s_shape, s_dtype), _like(dscale, c_shape, c_dtype), None, None, None, None
+        dx, dshift, dscale = _first_order_only((dx, _like(dshift, s_shape, s_dtype), _like(dscale, c_shape, c_dtype)),
+                                               dy, x, scale)
+        return dx, None, dshift, dscale, None, None, None, None
 
     @staticmethod
     def jvp(ctx, *tangents):
@@ -238,7 +259,8 @@ class GateResidualFunc(torch.autograd.Function):
     def backward(ctx, dout, *unused):
         h, gate = ctx.saved_tensors
         dh, dgate = gate_residual_bwd_raw(dout, h, gate)
-        return dout, None, dh, None, _like(dgate, *ctx.gate_meta), None
+        dh, dgate = _first_order_only((dh, _like(dgate, *ctx.gate_meta)), dout, h, gate)
+        return dout, None, dh, None, dgate, None
 
     @staticmethod
     def jvp(ctx, *tangents):

@@ -13,7 +13,7 @@
 //     rejects, CPU tensors) returns None, and the Python caller takes the general route, which also raises the exact errors.
 //
 // Semantics are those of the autograd.Functions in flash_attn_jvp.py, rms_norm.py and adaln.py: tangents are plain
-// inputs, backward differentiates the primal outputs only, tangent outputs carry no gradient.
+// inputs, backward differentiates the primal outputs only and once, tangent outputs carry no gradient.
 #include <ATen/ATen.h>
 #include <ATen/FuncTorchTLS.h>
 #include <ATen/autocast_mode.h>
@@ -154,6 +154,35 @@ bool needs_grad(std::initializer_list<const Tensor*> ts) {
   for (const Tensor* t : ts)
     if (t->defined() && t->requires_grad()) return true;
   return false;
+}
+
+// Gradients that a kernel's backward made cannot be differentiated again.  With create_graph they hang on this node, which
+// raises when a second derivative is asked for - as the registered ops of the general route do - instead of leaving it out.
+struct FirstOrderOnly : torch::autograd::Function<FirstOrderOnly> {
+  static variable_list forward(AutogradContext*, at::TensorList grads, at::TensorList /*sources*/) {
+    at::AutoDispatchBelowADInplaceOrView below_autograd;
+    variable_list out;
+    for (const Tensor& g : grads) out.push_back(g.detach());
+    return out;
+  }
+  static variable_list backward(AutogradContext*, variable_list) {
+    TORCH_CHECK(false, "dmf_b200 ops have no second derivatives");
+  }
+};
+
+// `grads` as a backward returns them, where they depend on `sources` (incoming gradient and saved tensors)
+variable_list first_order_only(variable_list grads, std::initializer_list<const Tensor*> sources) {
+  if (!needs_grad(sources)) return grads;
+  variable_list made, from;
+  for (const Tensor& g : grads)
+    if (g.defined()) made.push_back(g);
+  for (const Tensor* t : sources)
+    if (t->defined() && t->requires_grad()) from.push_back(*t);
+  const variable_list out = FirstOrderOnly::apply(at::TensorList(made), at::TensorList(from));
+  auto next = out.begin();
+  for (Tensor& g : grads)
+    if (g.defined()) g = *next++;
+  return grads;
 }
 
 // ---- attention ----------------------------------------------------------------------------------------------------------
@@ -310,14 +339,16 @@ struct AttnNode : torch::autograd::Function<AttnNode> {
     return dual ? variable_list{r.o, r.to} : variable_list{r.o};
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
-    at::AutoDispatchBelowADInplaceOrView below_autograd;
     const auto s = ctx->get_saved_variables();
-    if (!grads[0].defined()) {  // only the tangent output was used: it carries no gradient
-      return {at::zeros_like(s[0]), at::zeros_like(s[1]), at::zeros_like(s[2]), Tensor(), Tensor(), Tensor(), Tensor()};
-    }
-    variable_list g = attn_backward(grads[0], s[0], s[1], s[2], s[3], s[4], ctx->saved_data["scale"].toDouble());
+    variable_list g = backward_once(ctx, grads, s);
     g.resize(7);
-    return g;
+    return first_order_only(std::move(g), {&grads[0], &s[0], &s[1], &s[2]});
+  }
+  static variable_list backward_once(AutogradContext* ctx, const variable_list& grads, const variable_list& s) {
+    at::AutoDispatchBelowADInplaceOrView below_autograd;
+    if (!grads[0].defined())  // only the tangent output was used: it carries no gradient
+      return {at::zeros_like(s[0]), at::zeros_like(s[1]), at::zeros_like(s[2])};
+    return attn_backward(grads[0], s[0], s[1], s[2], s[3], s[4], ctx->saved_data["scale"].toDouble());
   }
 };
 
@@ -332,10 +363,13 @@ struct AttnPackedNode : torch::autograd::Function<AttnPackedNode> {
     return r.to.defined() ? variable_list{r.o, r.to} : variable_list{r.o};
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
-    at::AutoDispatchBelowADInplaceOrView below_autograd;
     const auto s = ctx->get_saved_variables();
-    if (!grads[0].defined()) return {at::zeros_like(s[0]), Tensor(), Tensor()};
-    return {attn_backward_packed(grads[0], s[0], s[1], s[2], ctx->saved_data["scale"].toDouble()), Tensor(), Tensor()};
+    return first_order_only({backward_once(ctx, grads, s), Tensor(), Tensor()}, {&grads[0], &s[0]});
+  }
+  static Tensor backward_once(AutogradContext* ctx, const variable_list& grads, const variable_list& s) {
+    at::AutoDispatchBelowADInplaceOrView below_autograd;
+    if (!grads[0].defined()) return at::zeros_like(s[0]);
+    return attn_backward_packed(grads[0], s[0], s[1], s[2], ctx->saved_data["scale"].toDouble());
   }
 };
 
@@ -460,8 +494,11 @@ struct RmsNode : torch::autograd::Function<RmsNode> {
     return r.ty.defined() ? variable_list{r.y, r.ty} : variable_list{r.y};
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
-    at::AutoDispatchBelowADInplaceOrView below_autograd;
     const auto s = ctx->get_saved_variables();
+    return first_order_only(backward_once(ctx, grads, s), {&grads[0], &s[0], &s[1]});
+  }
+  static variable_list backward_once(AutogradContext* ctx, const variable_list& grads, const variable_list& s) {
+    at::AutoDispatchBelowADInplaceOrView below_autograd;
     if (!grads[0].defined()) return {at::zeros_like(s[0]), Tensor(), at::zeros_like(s[1]), Tensor()};
     const c10::cuda::CUDAGuard device_guard(s[0].device());
     TORCH_CHECK(same_kind(s[0], grads[0]), "dmf_b200 RMS norm backward: unexpected gradient");
@@ -616,8 +653,11 @@ struct LnNode : torch::autograd::Function<LnNode> {
     return r.ty.defined() ? variable_list{r.y, r.ty} : variable_list{r.y};
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
-    at::AutoDispatchBelowADInplaceOrView below_autograd;
     const auto s = ctx->get_saved_variables();
+    return first_order_only(backward_once(ctx, grads, s), {&grads[0], &s[0], &s[1]});
+  }
+  static variable_list backward_once(AutogradContext* ctx, const variable_list& grads, const variable_list& s) {
+    at::AutoDispatchBelowADInplaceOrView below_autograd;
     const auto shift_shape = ctx->saved_data["shift_shape"].toIntVector();
     const auto shift_dtype = static_cast<at::ScalarType>(ctx->saved_data["shift_dtype"].toInt());
     if (!grads[0].defined())
@@ -717,8 +757,14 @@ struct GateNode : torch::autograd::Function<GateNode> {
     return r.ty.defined() ? variable_list{r.y, r.ty} : variable_list{r.y};
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
-    at::AutoDispatchBelowADInplaceOrView below_autograd;
     const auto s = ctx->get_saved_variables();
+    variable_list g = first_order_only(backward_once(ctx, grads, s), {&grads[0], &s[0], &s[1]});
+    g[0] = grads[0];  // x's gradient is the incoming one, with its graph
+    return g;
+  }
+  // all but x's gradient
+  static variable_list backward_once(AutogradContext* ctx, const variable_list& grads, const variable_list& s) {
+    at::AutoDispatchBelowADInplaceOrView below_autograd;
     if (!grads[0].defined())
       return {Tensor(), Tensor(), at::zeros_like(s[0]), Tensor(), at::zeros_like(s[1]), Tensor()};
     const c10::cuda::CUDAGuard device_guard(s[0].device());
@@ -738,7 +784,7 @@ struct GateNode : torch::autograd::Function<GateNode> {
     const int st = dmf_gate_residual_bwd(&a);
     TORCH_CHECK(st == DMF_ATTN_OK, "dmf_attn: ", dmf_attn_status_string(st));
     g_launches.fetch_add(2, std::memory_order_relaxed);
-    return {grads[0], Tensor(), dh, Tensor(), ada_mod_grad(dgate, s[1]), Tensor()};
+    return {Tensor(), Tensor(), dh, Tensor(), ada_mod_grad(dgate, s[1]), Tensor()};
   }
 };
 

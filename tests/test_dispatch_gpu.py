@@ -48,3 +48,18 @@ def test_a_traced_call_replays_on_new_inputs(op):
     traced = torch.jit.trace(fn, tuple(args))
     new = _case(op, seed=7)[1]
     assert torch.equal(traced(*new), fn(*new))
+
+
+@pytest.mark.parametrize("op", ("attn", "packed", "rms", "ln", "gate"))
+def test_second_derivatives_are_refused(op):
+    """Neither the kernels nor their host code compute them: a loss that asks for one must not get a number without it."""
+    fn, args = _case(op)
+    args = [a.requires_grad_(True) for a in args]
+    out = fn(*args)
+    first = torch.autograd.grad(out, args, torch.ones_like(out), create_graph=True)
+    plain = torch.autograd.grad(fn(*args), args, torch.ones_like(out))
+    assert all(torch.equal(a, b) for a, b in zip(first, plain, strict=True))
+    which = {"gate": 2}.get(op, 0)                  # (the gradient of the gate's x is the incoming one: linear)
+    loss = (first[which].float() * args[which].float()).sum()
+    with pytest.raises(RuntimeError):
+        torch.autograd.grad(loss, args, allow_unused=True)
