@@ -854,6 +854,18 @@ PairOut gelu_forward(const Tensor& x_, const Tensor& tx_) {
   return r;
 }
 
+// gelu'(x) dy by the kernel
+Tensor gelu_gradient(const Tensor& x_, const Tensor& dy_) {
+  const c10::cuda::CUDAGuard device_guard(x_.device());
+  TORCH_CHECK(dy_.sizes() == x_.sizes() && dy_.scalar_type() == x_.scalar_type() && dy_.device() == x_.device(),
+              "dmf_b200 GELU backward: unexpected gradient");
+  const Tensor x = gelu_flat(x_), dy = gelu_flat(dy_);
+  const Tensor dx = at::empty(x.sizes(), x.options());
+  const int st = gelu_launch(x, dy, Tensor(), dx);
+  TORCH_CHECK(st == DMF_ATTN_OK, "dmf_attn: ", dmf_attn_status_string(st));
+  return dx;
+}
+
 struct GeluNode : torch::autograd::Function<GeluNode> {
   static variable_list forward(AutogradContext* ctx, const Tensor& x, const std::optional<Tensor>& tx) {
     at::AutoDispatchBelowADInplaceOrView below_autograd;
@@ -864,18 +876,11 @@ struct GeluNode : torch::autograd::Function<GeluNode> {
     return r.ty.defined() ? variable_list{r.y, r.ty} : variable_list{r.y};
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
-    at::AutoDispatchBelowADInplaceOrView below_autograd;
     const auto s = ctx->get_saved_variables();
     if (!grads[0].defined()) return {at::zeros_like(s[0]), Tensor()};
-    const c10::cuda::CUDAGuard device_guard(s[0].device());
-    TORCH_CHECK(grads[0].sizes() == s[0].sizes() && grads[0].scalar_type() == s[0].scalar_type() &&
-                    grads[0].device() == s[0].device(),
-                "dmf_b200 GELU backward: unexpected gradient");
-    const Tensor x = gelu_flat(s[0]), dy = gelu_flat(grads[0]);
-    const Tensor dx = at::empty(x.sizes(), x.options());
-    const int st = gelu_launch(x, dy, Tensor(), dx);
-    TORCH_CHECK(st == DMF_ATTN_OK, "dmf_attn: ", dmf_attn_status_string(st));
-    return {dx, Tensor()};
+    if (needs_grad({&grads[0], &s[0]})) return {at::gelu_backward(grads[0], s[0], "tanh"), Tensor()};  // differentiable again
+    at::AutoDispatchBelowADInplaceOrView below_autograd;
+    return {gelu_gradient(s[0], grads[0]), Tensor()};
   }
 };
 

@@ -63,3 +63,15 @@ def test_second_derivatives_are_refused(op):
     loss = (first[which].float() * args[which].float()).sum()
     with pytest.raises(RuntimeError):
         torch.autograd.grad(loss, args, allow_unused=True)
+
+
+def test_gelu_has_its_second_derivative():
+    lib = lambda x: torch.nn.functional.gelu(x, approximate="tanh")
+    x, dy, v = (_randn(3, 50, 40, seed=s) for s in (1, 2, 3))
+    res = []
+    for fn in (adaln.gelu, lib):
+        a, g = x.clone().requires_grad_(True), dy.clone().requires_grad_(True)
+        first, = torch.autograd.grad(fn(a), a, g, create_graph=True)
+        res.append((first, *torch.autograd.grad(first, (a, g), v)))
+    for a, b in zip(*res, strict=True):
+        assert torch.equal(a, b)
