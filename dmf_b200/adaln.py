@@ -318,8 +318,8 @@ def gate_residual(x: torch.Tensor, gate: torch.Tensor, h: torch.Tensor) -> torch
 
 def gelu(x: torch.Tensor) -> torch.Tensor:
     """GELU in its tanh form (the block's MLP), as one kernel for 16-bit CUDA tensors; a dual tensor in gives a dual tensor
-    out, and backward differentiates the primal output only.  Everything else (other types and devices, transforms the
-    native path does not take) is ``torch.nn.functional.gelu``, the same function."""
+    out.  Everything else (other types and devices, transforms the native path does not take) is
+    ``torch.nn.functional.gelu``: the same function, with the same values, gradients and second derivatives."""
     if not torch.compiler.is_compiling():
         out = _native.gelu(x)
         if out is not None:

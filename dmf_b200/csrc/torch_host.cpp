@@ -13,7 +13,8 @@
 //     rejects, CPU tensors) returns None, and the Python caller takes the general route, which also raises the exact errors.
 //
 // Semantics are those of the autograd.Functions in flash_attn_jvp.py, rms_norm.py and adaln.py: tangents are plain
-// inputs, backward differentiates the primal outputs only and once, tangent outputs carry no gradient.
+// inputs, backward differentiates the primal outputs only and once, tangent outputs carry no gradient (GELU, which stands in
+// for a library function, excepted).
 #include <ATen/ATen.h>
 #include <ATen/FuncTorchTLS.h>
 #include <ATen/autocast_mode.h>
@@ -22,6 +23,7 @@
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/autograd.h>
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/jit/frontend/tracer.h>
 #include <torch/extension.h>
@@ -866,21 +868,40 @@ Tensor gelu_gradient(const Tensor& x_, const Tensor& dy_) {
   return dx;
 }
 
+// Unlike the other ops' nodes this one differentiates its tangent output too, as the library's GELU does: rarely wanted
+// (a loss that does not detach the tangent), and left to differentiable library calls.
 struct GeluNode : torch::autograd::Function<GeluNode> {
   static variable_list forward(AutogradContext* ctx, const Tensor& x, const std::optional<Tensor>& tx) {
     at::AutoDispatchBelowADInplaceOrView below_autograd;
     PairOut r = gelu_forward(x, value_of(tx));
     if (r.status != DMF_ATTN_OK) throw RejectedError();
-    ctx->save_for_backward({x});
+    ctx->save_for_backward(tx.has_value() ? variable_list{x, *tx} : variable_list{x});
     ctx->set_materialize_grads(false);
     return r.ty.defined() ? variable_list{r.y, r.ty} : variable_list{r.y};
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto s = ctx->get_saved_variables();
-    if (!grads[0].defined()) return {at::zeros_like(s[0]), Tensor()};
-    if (needs_grad({&grads[0], &s[0]})) return {at::gelu_backward(grads[0], s[0], "tanh"), Tensor()};  // differentiable again
-    at::AutoDispatchBelowADInplaceOrView below_autograd;
-    return {gelu_gradient(s[0], grads[0]), Tensor()};
+    Tensor dx, dtx;
+    if (grads[0].defined()) {
+      if (needs_grad({&grads[0], &s[0]})) {
+        dx = at::gelu_backward(grads[0], s[0], "tanh");  // differentiable again
+      } else {
+        at::AutoDispatchBelowADInplaceOrView below_autograd;
+        dx = gelu_gradient(s[0], grads[0]);
+      }
+    }
+    if (grads.size() > 1 && grads[1].defined()) {  // ty = gelu'(x) tx
+      const bool create_graph = at::GradMode::is_enabled();
+      const at::AutoGradMode with_graph(true);
+      const Tensor x = create_graph ? s[0].view_as(s[0]) : s[0].detach(), tx = create_graph ? s[1].view_as(s[1]) : s[1].detach();
+      if (!x.requires_grad()) x.set_requires_grad(true);
+      if (!tx.requires_grad()) tx.set_requires_grad(true);
+      const Tensor ty = at::gelu_backward(tx, x, "tanh");
+      const variable_list g = torch::autograd::grad({ty}, {x, tx}, {grads[1]}, /*retain_graph=*/std::nullopt, create_graph);
+      dx = dx.defined() ? dx + g[0] : g[0];
+      dtx = g[1];
+    }
+    return {dx, dtx};
   }
 };
 
@@ -893,7 +914,7 @@ std::optional<Tensor> gelu(const Tensor& x_) {
     return std::nullopt;
   std::optional<BelowTransform> guard(std::in_place, route.jvp);
   Tensor y, ty;
-  if (needs_grad({&x.p})) {
+  if (needs_grad({&x.p, &x.t})) {
     try {
       variable_list out = GeluNode::apply(x.p, maybe(x.t));
       y = out[0];

@@ -75,3 +75,18 @@ def test_gelu_has_its_second_derivative():
         res.append((first, *torch.autograd.grad(first, (a, g), v)))
     for a, b in zip(*res, strict=True):
         assert torch.equal(a, b)
+
+
+def test_gelu_tangent_carries_its_gradient():
+    """The library's GELU differentiates its tangent in reverse; so does this one."""
+    lib = lambda x: torch.nn.functional.gelu(x, approximate="tanh")
+    x, t, dy, dty = (_randn(3, 50, 40, seed=s) for s in (1, 2, 3, 4))
+    res = []
+    for fn in (adaln.gelu, lib):
+        a, ta = x.clone().requires_grad_(True), t.clone().requires_grad_(True)
+        y, ty = torch.func.jvp(fn, (a,), (ta,))
+        res.append(torch.autograd.grad((y, ty), (a, ta), (dy, dty), retain_graph=True)
+                   + torch.autograd.grad(ty, (a, ta), dty))
+    for a, b in zip(*res, strict=True):
+        # the primal's and the tangent's share of the gradient are added in 16 bits, in either order: half an ulp of each
+        assert torch.allclose(a.float(), b.float(), rtol=2.0 ** -7, atol=2.0 ** -7)
