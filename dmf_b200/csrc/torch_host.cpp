@@ -18,6 +18,7 @@
 #include <ATen/ATen.h>
 #include <ATen/FuncTorchTLS.h>
 #include <ATen/autocast_mode.h>
+#include <ATen/core/dispatch/Dispatcher.h>
 #include <ATen/functorch/DynamicLayer.h>
 #include <ATen/functorch/TensorWrapper.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
@@ -58,8 +59,8 @@ bool plain_cuda(const Tensor& t) {
                                      c10::DispatchKey::ZeroTensor, c10::DispatchKey::Negative,
                                      c10::DispatchKey::Conjugate, c10::DispatchKey::Functionalize,
                                      c10::DispatchKey::FuncTorchBatched, c10::DispatchKey::BatchedNestedTensor,
-                                     c10::DispatchKey::FuncTorchGradWrapper});
-  return t.defined() && t.is_cuda() && t.layout() == at::kStrided && (t.key_set() & odd).empty();
+                                     c10::DispatchKey::Batched, c10::DispatchKey::FuncTorchGradWrapper});
+  return t.defined() && t.is_cuda() && t.layout() == at::kStrided && (t.key_set() & odd).empty() && t.has_storage();
 }
 
 // Where the call stands: no transform, or one JVP level `level` whose wrappers are to be taken off and put on again.
@@ -185,6 +186,14 @@ variable_list first_order_only(variable_list grads, std::initializer_list<const 
   for (Tensor& g : grads)
     if (g.defined()) g = *next++;
   return grads;
+}
+
+// A gradient that is not a plain tensor (is_grads_batched, a subclass) goes to the registered op of the general route, which
+// the dispatcher can unwrap.
+template <typename R, typename... Args>
+R registered_op(const char* name, const Args&... args) {
+  const auto op = c10::Dispatcher::singleton().findSchemaOrThrow(name, "");
+  return op.template typed<R(Args...)>().call(args...);
 }
 
 // ---- attention ----------------------------------------------------------------------------------------------------------
@@ -342,6 +351,11 @@ struct AttnNode : torch::autograd::Function<AttnNode> {
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto s = ctx->get_saved_variables();
+    if (grads[0].defined() && !plain_cuda(grads[0])) {
+      const auto [dq, dk, dv] = registered_op<std::tuple<Tensor, Tensor, Tensor>>(
+          "dmf_b200::attn_bwd", grads[0], s[0], s[1], s[2], s[3], s[4], ctx->saved_data["scale"].toDouble());
+      return {dq, dk, dv, Tensor(), Tensor(), Tensor(), Tensor()};
+    }
     variable_list g = backward_once(ctx, grads, s);
     g.resize(7);
     return first_order_only(std::move(g), {&grads[0], &s[0], &s[1], &s[2]});
@@ -366,6 +380,9 @@ struct AttnPackedNode : torch::autograd::Function<AttnPackedNode> {
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto s = ctx->get_saved_variables();
+    if (grads[0].defined() && !plain_cuda(grads[0]))
+      return {registered_op<Tensor>("dmf_b200::attn_bwd_qkvpacked", grads[0], s[0], s[1], s[2],
+                                    ctx->saved_data["scale"].toDouble()), Tensor(), Tensor()};
     return first_order_only({backward_once(ctx, grads, s), Tensor(), Tensor()}, {&grads[0], &s[0]});
   }
   static Tensor backward_once(AutogradContext* ctx, const variable_list& grads, const variable_list& s) {
@@ -497,6 +514,11 @@ struct RmsNode : torch::autograd::Function<RmsNode> {
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto s = ctx->get_saved_variables();
+    if (grads[0].defined() && !plain_cuda(grads[0])) {
+      const auto [dx, dw] = registered_op<std::tuple<Tensor, Tensor>>("dmf_b200::rmsnorm_bwd", grads[0], s[0], s[1],
+                                                                      ctx->saved_data["eps"].toDouble());
+      return {dx, Tensor(), dw.to(s[1].scalar_type()), Tensor()};
+    }
     return first_order_only(backward_once(ctx, grads, s), {&grads[0], &s[0], &s[1]});
   }
   static variable_list backward_once(AutogradContext* ctx, const variable_list& grads, const variable_list& s) {
@@ -666,6 +688,7 @@ struct LnNode : torch::autograd::Function<LnNode> {
       return {at::zeros_like(s[0]), Tensor(), at::zeros(shift_shape, s[1].options().dtype(shift_dtype)),
               at::zeros_like(s[1]), Tensor(), Tensor(), Tensor(), Tensor()};
     const c10::cuda::CUDAGuard device_guard(s[0].device());
+    TORCH_CHECK(plain_cuda(grads[0]), "dmf_b200 LayerNorm-modulate backward: unexpected gradient");
     const Tensor x = ada_rows(s[0]), dy = ada_rows(grads[0]);
     TORCH_CHECK(dy.sizes() == x.sizes() && ada_pair_ok(x.scalar_type(), dy.scalar_type()),
                 "dmf_b200 LayerNorm-modulate backward: unexpected gradient");
@@ -770,6 +793,7 @@ struct GateNode : torch::autograd::Function<GateNode> {
     if (!grads[0].defined())
       return {Tensor(), Tensor(), at::zeros_like(s[0]), Tensor(), at::zeros_like(s[1]), Tensor()};
     const c10::cuda::CUDAGuard device_guard(s[0].device());
+    TORCH_CHECK(plain_cuda(grads[0]), "dmf_b200 gate-residual backward: unexpected gradient");
     const Tensor dout = ada_rows(grads[0]), h = ada_rows(s[0]);
     TORCH_CHECK(dout.sizes() == h.sizes() && ada_pair_ok(dout.scalar_type(), h.scalar_type()),
                 "dmf_b200 gate-residual backward: unexpected gradient");
@@ -883,8 +907,8 @@ struct GeluNode : torch::autograd::Function<GeluNode> {
     const auto s = ctx->get_saved_variables();
     Tensor dx, dtx;
     if (grads[0].defined()) {
-      if (needs_grad({&grads[0], &s[0]})) {
-        dx = at::gelu_backward(grads[0], s[0], "tanh");  // differentiable again
+      if (needs_grad({&grads[0], &s[0]}) || !plain_cuda(grads[0])) {
+        dx = at::gelu_backward(grads[0], s[0], "tanh");  // differentiable again, and for batched gradients
       } else {
         at::AutoDispatchBelowADInplaceOrView below_autograd;
         dx = gelu_gradient(s[0], grads[0]);

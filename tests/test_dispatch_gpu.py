@@ -90,3 +90,15 @@ def test_gelu_tangent_carries_its_gradient():
     for a, b in zip(*res, strict=True):
         # the primal's and the tangent's share of the gradient are added in 16 bits, in either order: half an ulp of each
         assert torch.allclose(a.float(), b.float(), rtol=2.0 ** -7, atol=2.0 ** -7)
+
+
+@pytest.mark.parametrize("op", ("attn", "packed", "rms", "gelu"))
+def test_batched_gradients(op):
+    fn, args = _case(op)
+    args = [a.requires_grad_(True) for a in args]
+    out = fn(*args)
+    douts = torch.stack([_randn(*out.shape, seed=s) for s in (1, 2, 3)])
+    batched = torch.autograd.grad(out, args, douts, is_grads_batched=True, retain_graph=True)
+    for i, dout in enumerate(douts):
+        for a, b in zip(batched, torch.autograd.grad(out, args, dout, retain_graph=True), strict=True):
+            assert torch.equal(a[i], b)
