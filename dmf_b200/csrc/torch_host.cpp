@@ -778,20 +778,22 @@ struct GateNode : torch::autograd::Function<GateNode> {
     PairOut r = gate_forward(x, value_of(tx), h, value_of(th), gate, value_of(tgate));
     if (r.status != DMF_ATTN_OK) throw RejectedError();
     ctx->save_for_backward({h, gate});
+    ctx->saved_data["x_dtype"] = static_cast<int64_t>(x.scalar_type());
     ctx->set_materialize_grads(false);
     return r.ty.defined() ? variable_list{r.y, r.ty} : variable_list{r.y};
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto s = ctx->get_saved_variables();
     variable_list g = first_order_only(backward_once(ctx, grads, s), {&grads[0], &s[0], &s[1]});
-    g[0] = grads[0];  // x's gradient is the incoming one, with its graph
+    if (grads[0].defined()) g[0] = grads[0];  // x's gradient is the incoming one, with its graph
     return g;
   }
-  // all but x's gradient
+  // all but x's gradient, which is the incoming one (zero where only the tangent output was used)
   static variable_list backward_once(AutogradContext* ctx, const variable_list& grads, const variable_list& s) {
     at::AutoDispatchBelowADInplaceOrView below_autograd;
     if (!grads[0].defined())
-      return {Tensor(), Tensor(), at::zeros_like(s[0]), Tensor(), at::zeros_like(s[1]), Tensor()};
+      return {at::zeros_like(s[0], at::TensorOptions().dtype(static_cast<at::ScalarType>(ctx->saved_data["x_dtype"].toInt()))),
+              Tensor(), at::zeros_like(s[0]), Tensor(), at::zeros_like(s[1]), Tensor()};
     const c10::cuda::CUDAGuard device_guard(s[0].device());
     TORCH_CHECK(plain_cuda(grads[0]), "dmf_b200 gate-residual backward: unexpected gradient");
     const Tensor dout = ada_rows(grads[0]), h = ada_rows(s[0]);

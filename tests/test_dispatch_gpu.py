@@ -102,3 +102,19 @@ def test_batched_gradients(op):
     for i, dout in enumerate(douts):
         for a, b in zip(batched, torch.autograd.grad(out, args, dout, retain_graph=True), strict=True):
             assert torch.equal(a[i], b)
+
+
+@pytest.mark.parametrize("op", ALL)
+def test_gradients_of_the_tangent_alone(op):
+    """Backward differentiates the primal output; the gradient that the tangent output brings is zero, for every input."""
+    if op == "gelu":
+        pytest.skip("differentiates its tangent")
+    fn, args = _case(op)
+    args = [a.requires_grad_(True) for a in args]
+    if op == "rms":
+        fn_, w = fn, args[1]
+        _, tangent = torch.func.jvp(lambda x: fn_(x, w), (args[0],), (torch.ones_like(args[0]),))
+    else:
+        _, tangent = torch.func.jvp(fn, tuple(args), tuple(torch.ones_like(a) for a in args))
+    for a, g in zip(args, torch.autograd.grad(tangent.float().sum(), args), strict=True):
+        assert g.shape == a.shape and g.dtype == a.dtype and not g.any()
