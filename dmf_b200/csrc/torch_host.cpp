@@ -406,7 +406,7 @@ std::optional<Tensor> attn_func(const Tensor& q_, const Tensor& k_, const Tensor
     }
   const double scale = softmax_scale.has_value() ? *softmax_scale : std::pow(static_cast<double>(q.p.size(3)), -0.5);
   Tensor o, to;
-  if (needs_grad({&q.p, &k.p, &v.p})) {
+  if (needs_grad({&q.p, &k.p, &v.p, &q.t, &k.t, &v.t})) {
     try {
       variable_list out = AttnNode::apply(q.p, k.p, v.p, maybe(q.t), maybe(k.t), maybe(v.t), scale);
       o = out[0];
@@ -438,7 +438,7 @@ std::optional<Tensor> attn_qkvpacked(const Tensor& qkv_, std::optional<double> s
   std::optional<BelowTransform> guard(std::in_place, route.jvp);
   const double scale = softmax_scale.has_value() ? *softmax_scale : std::pow(static_cast<double>(x.p.size(4)), -0.5);
   Tensor o, to;
-  if (needs_grad({&x.p})) {
+  if (needs_grad({&x.p, &x.t})) {
     try {
       variable_list out = AttnPackedNode::apply(x.p, maybe(x.t), scale);
       o = out[0];
@@ -557,7 +557,7 @@ std::optional<Tensor> rms_norm(const Tensor& x_, const Tensor& weight_, double e
   if (x.t.defined() && (x.t.sizes() != x.p.sizes() || !same_kind(x.p, x.t))) return std::nullopt;
   std::optional<BelowTransform> guard(std::in_place, route.jvp);
   Tensor y, ty;
-  if (needs_grad({&x.p, &w.p})) {
+  if (needs_grad({&x.p, &x.t, &w.p})) {
     try {
       variable_list out = RmsNode::apply(x.p, maybe(x.t), w.p, eps);
       y = out[0];
@@ -728,7 +728,7 @@ std::optional<Tensor> ln_modulate(const Tensor& x_, const Tensor& shift_, const 
   if (dual && !x.t.defined()) x.t = at::zeros_like(x.p);
   if (dual && x.t.sizes() != x.p.sizes()) return std::nullopt;
   Tensor y, ty;
-  if (needs_grad({&x.p, &shift.p, &scale.p})) {
+  if (needs_grad({&x.p, &shift.p, &scale.p, &x.t, &shift.t, &scale.t})) {
     try {
       variable_list out = LnNode::apply(x.p, maybe(x.t), shift.p, scale.p, maybe(shift.t), maybe(scale.t), eps,
                                         static_cast<int64_t>(narrow));
@@ -829,7 +829,7 @@ std::optional<Tensor> gate_residual(const Tensor& x_, const Tensor& gate_, const
     if (!ada_mod_fits(*m, x.p)) return std::nullopt;
   std::optional<BelowTransform> guard(std::in_place, route.jvp);
   Tensor y, ty;
-  if (needs_grad({&x.p, &h.p, &gate.p})) {
+  if (needs_grad({&x.p, &h.p, &gate.p, &x.t, &h.t, &gate.t})) {
     try {
       variable_list out = GateNode::apply(x.p, maybe(x.t), h.p, maybe(h.t), gate.p, maybe(gate.t));
       y = out[0];

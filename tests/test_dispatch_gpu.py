@@ -118,3 +118,16 @@ def test_gradients_of_the_tangent_alone(op):
         _, tangent = torch.func.jvp(fn, tuple(args), tuple(torch.ones_like(a) for a in args))
     for a, g in zip(args, torch.autograd.grad(tangent.float().sum(), args), strict=True):
         assert g.shape == a.shape and g.dtype == a.dtype and not g.any()
+
+
+@pytest.mark.parametrize("op", ("attn", "packed", "rms", "ln", "gate"))
+def test_a_tangent_that_requires_grad_keeps_the_graph(op):
+    """Outputs of inputs without gradients belong to a graph when a tangent does, and its gradient is None."""
+    fn, args = _case(op)
+    tangents = [torch.ones_like(a).requires_grad_(True) for a in args]
+    if op == "rms":
+        fn_, w = fn, args[1]
+        fn, args, tangents = (lambda x: fn_(x, w)), args[:1], tangents[:1]
+    out, _ = torch.func.jvp(fn, tuple(args), tuple(tangents))
+    assert out.requires_grad
+    assert torch.autograd.grad(out.float().sum(), tangents, allow_unused=True) == (None,) * len(tangents)
