@@ -236,6 +236,11 @@ bool attn_inputs_ok(const Tensor& q, const Tensor& k, const Tensor& v) {
          g_status_word[q.get_device()].load(std::memory_order_acquire) != nullptr;
 }
 
+bool lse_ok(const Tensor& lse, const Tensor& o) {
+  return lse.scalar_type() == at::kFloat && lse.device() == o.device() &&
+         lse.sizes() == at::IntArrayRef({o.size(0), o.size(2), o.size(1)});
+}
+
 struct AttnOut {
   Tensor o, to, lse;
   int status = DMF_ATTN_OK;
@@ -292,6 +297,11 @@ AttnOut attn_forward_packed(const Tensor& qkv_, const Tensor& tqkv_, double scal
   return attn_launch(&a, qkv, true);
 }
 
+// Saved-tensor hooks hand back whatever they like: layouts are put right like those of inputs, anything else must be as saved.
+void check_saved(bool as_saved) {
+  TORCH_CHECK(as_saved, "dmf_b200 backward: a saved tensor came back with another type, shape or device");
+}
+
 // workspace and launch of a backward, with the tensors of `a` filled in
 void attn_launch_bwd(dmf_attn_bwd_args* a, const Tensor& like, const Tensor& lse) {
   const size_t bytes = dmf_attn_bwd_workspace_bytes(a->batch, a->seqlen_q, a->seqlen_kv, a->heads, a->head_dim);
@@ -304,11 +314,13 @@ void attn_launch_bwd(dmf_attn_bwd_args* a, const Tensor& like, const Tensor& lse
   g_launches.fetch_add(2, std::memory_order_relaxed);
 }
 
-variable_list attn_backward(const Tensor& dout_, const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& o,
-                            const Tensor& lse, double scale) {
+variable_list attn_backward(const Tensor& dout_, const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& o_,
+                            const Tensor& lse_, double scale) {
+  for (const Tensor* t : {&q_, &k_, &v_, &o_, &lse_}) check_saved(plain_cuda(*t));
+  check_saved(attn_inputs_ok(q_, k_, v_) && same_kind(q_, o_) && o_.sizes() == q_.sizes() && lse_ok(lse_, o_));
   const c10::cuda::CUDAGuard device_guard(q_.device());
-  TORCH_CHECK(same_kind(q_, dout_) && dout_.sizes() == o.sizes(), "dmf_b200 attention backward: unexpected gradient");
-  const Tensor dout = prep(dout_), q = prep(q_), k = prep(k_), v = prep(v_);
+  TORCH_CHECK(same_kind(q_, dout_) && dout_.sizes() == o_.sizes(), "dmf_b200 attention backward: unexpected gradient");
+  const Tensor dout = prep(dout_), q = prep(q_), k = prep(k_), v = prep(v_), o = prep(o_), lse = lse_.contiguous();
   variable_list grads = {at::empty(q.sizes(), q.options()), at::empty(k.sizes(), q.options()), at::empty(v.sizes(), q.options())};
   dmf_attn_bwd_args a = {};
   attn_sizes(&a, q, q.size(0), q.size(1), k.size(1), q.size(2), q.size(3), scale);
@@ -319,11 +331,15 @@ variable_list attn_backward(const Tensor& dout_, const Tensor& q_, const Tensor&
 }
 
 // one (B, L, 3, H, D) gradient
-Tensor attn_backward_packed(const Tensor& dout_, const Tensor& qkv_, const Tensor& o, const Tensor& lse, double scale) {
+Tensor attn_backward_packed(const Tensor& dout_, const Tensor& qkv_, const Tensor& o_, const Tensor& lse_, double scale) {
+  for (const Tensor* t : {&qkv_, &o_, &lse_}) check_saved(plain_cuda(*t));
+  check_saved(qkv_.dim() == 5 && qkv_.size(2) == 3 && attn_dtype(qkv_.scalar_type()) >= 0 &&
+              o_.scalar_type() == qkv_.scalar_type() && o_.device() == qkv_.device() &&
+              o_.sizes() == at::IntArrayRef({qkv_.size(0), qkv_.size(1), qkv_.size(3), qkv_.size(4)}) && lse_ok(lse_, o_));
   const c10::cuda::CUDAGuard device_guard(qkv_.device());
-  TORCH_CHECK(dout_.scalar_type() == o.scalar_type() && dout_.device() == o.device() && dout_.sizes() == o.sizes(),
+  TORCH_CHECK(dout_.scalar_type() == o_.scalar_type() && dout_.device() == o_.device() && dout_.sizes() == o_.sizes(),
               "dmf_b200 attention backward: unexpected gradient");
-  const Tensor dout = prep(dout_), qkv = packed_ok(qkv_) ? qkv_ : qkv_.contiguous();
+  const Tensor dout = prep(dout_), o = prep(o_), lse = lse_.contiguous(), qkv = packed_ok(qkv_) ? qkv_ : qkv_.contiguous();
   const Tensor grad = at::empty(qkv.sizes(), qkv.options());
   dmf_attn_bwd_args a = {};
   attn_sizes(&a, qkv, qkv.size(0), qkv.size(1), qkv.size(1), qkv.size(3), qkv.size(4), scale);
@@ -524,8 +540,9 @@ struct RmsNode : torch::autograd::Function<RmsNode> {
   static variable_list backward_once(AutogradContext* ctx, const variable_list& grads, const variable_list& s) {
     at::AutoDispatchBelowADInplaceOrView below_autograd;
     if (!grads[0].defined()) return {at::zeros_like(s[0]), Tensor(), at::zeros_like(s[1]), Tensor()};
+    check_saved(plain_cuda(s[0]) && s[0].dim() == 4 && attn_dtype(s[0].scalar_type()) >= 0 && s[1].numel() == s[0].size(3));
     const c10::cuda::CUDAGuard device_guard(s[0].device());
-    TORCH_CHECK(same_kind(s[0], grads[0]), "dmf_b200 RMS norm backward: unexpected gradient");
+    TORCH_CHECK(same_kind(s[0], grads[0]) && s[0].sizes() == grads[0].sizes(), "dmf_b200 RMS norm backward: unexpected gradient");
     const Tensor x = prep(s[0]), dy = prep(grads[0]), w = rms_weight(s[1], x);
     const int64_t D = x.size(3);
     const Tensor dx = at::empty(x.sizes(), x.options());
@@ -687,6 +704,7 @@ struct LnNode : torch::autograd::Function<LnNode> {
     if (!grads[0].defined())
       return {at::zeros_like(s[0]), Tensor(), at::zeros(shift_shape, s[1].options().dtype(shift_dtype)),
               at::zeros_like(s[1]), Tensor(), Tensor(), Tensor(), Tensor()};
+    check_saved(plain_cuda(s[0]) && plain_cuda(s[1]) && s[0].dim() == 3 && ada_mod_fits(s[1], s[0]));
     const c10::cuda::CUDAGuard device_guard(s[0].device());
     TORCH_CHECK(plain_cuda(grads[0]), "dmf_b200 LayerNorm-modulate backward: unexpected gradient");
     const Tensor x = ada_rows(s[0]), dy = ada_rows(grads[0]);
@@ -794,6 +812,7 @@ struct GateNode : torch::autograd::Function<GateNode> {
     if (!grads[0].defined())
       return {at::zeros_like(s[0], at::TensorOptions().dtype(static_cast<at::ScalarType>(ctx->saved_data["x_dtype"].toInt()))),
               Tensor(), at::zeros_like(s[0]), Tensor(), at::zeros_like(s[1]), Tensor()};
+    check_saved(plain_cuda(s[0]) && plain_cuda(s[1]) && s[0].dim() == 3 && ada_mod_fits(s[1], s[0]));
     const c10::cuda::CUDAGuard device_guard(s[0].device());
     TORCH_CHECK(plain_cuda(grads[0]), "dmf_b200 gate-residual backward: unexpected gradient");
     const Tensor dout = ada_rows(grads[0]), h = ada_rows(s[0]);
@@ -884,6 +903,7 @@ PairOut gelu_forward(const Tensor& x_, const Tensor& tx_) {
 
 // gelu'(x) dy by the kernel
 Tensor gelu_gradient(const Tensor& x_, const Tensor& dy_) {
+  check_saved(plain_cuda(x_) && attn_dtype(x_.scalar_type()) >= 0);
   const c10::cuda::CUDAGuard device_guard(x_.device());
   TORCH_CHECK(dy_.sizes() == x_.sizes() && dy_.scalar_type() == x_.scalar_type() && dy_.device() == x_.device(),
               "dmf_b200 GELU backward: unexpected gradient");

@@ -131,3 +131,22 @@ def test_a_tangent_that_requires_grad_keeps_the_graph(op):
     out, _ = torch.func.jvp(fn, tuple(args), tuple(tangents))
     assert out.requires_grad
     assert torch.autograd.grad(out.float().sum(), tangents, allow_unused=True) == (None,) * len(tangents)
+
+
+@pytest.mark.parametrize("op", ALL)
+def test_saved_tensors_in_another_layout(op):
+    """A saved-tensor hook may hand back equal values with other strides."""
+    fn, args = _case(op)
+    args = [a.requires_grad_(True) for a in args]
+    other = lambda t: t.transpose(0, -1).clone(memory_format=torch.contiguous_format).transpose(0, -1) if t.dim() > 1 else t.clone()
+    dout = torch.ones_like(fn(*args))
+    plain = torch.autograd.grad(fn(*args), args, dout)
+    with torch.autograd.graph.saved_tensors_hooks(other, lambda t: t):
+        out = fn(*args)
+    for a, b in zip(torch.autograd.grad(out, args, dout), plain, strict=True):
+        assert torch.equal(a, b)
+    # ... but a tensor on another device is refused
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t.cpu(), lambda t: t):
+        out = fn(*args)
+    with pytest.raises((RuntimeError, ValueError)):
+        torch.autograd.grad(out, args, dout)
