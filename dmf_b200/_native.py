@@ -1,6 +1,9 @@
 """The native host path (csrc/torch_host.cpp): one C++ call per op for plain CUDA tensors, with or without autograd and under
 one ``torch.func.jvp``.  Its functions return None for everything else, and the caller takes the general route.
 
+``takes`` comes before them: what torch.compile traces, and tensors or modes with a __torch_function__ of their own, have to see
+the ops of the general route.
+
 With DMF_ATTN_CHECK=1 (which reads the device status word back after every call) every function returns None.
 """
 
@@ -9,8 +12,24 @@ from __future__ import annotations
 import importlib.util
 import os
 
+import torch
+from torch.overrides import _get_current_function_mode_stack, has_torch_function
+from torch.utils._device import DeviceContext
+
 from . import _lib
 from . import build as _build
+
+
+def takes(*tensors) -> bool:
+    """Whether a call on these tensors may go past torch's Python-level dispatch."""
+    if torch.compiler.is_compiling():
+        return False
+    if not has_torch_function(tensors):
+        return True
+    # `with torch.device(...)` and set_default_device are function modes too, but concern factory functions only
+    return (all(type(m) is DeviceContext for m in _get_current_function_mode_stack())
+            and all(type(t) is torch.Tensor or type(t).__torch_function__ is torch._C._disabled_torch_function_impl
+                    for t in tensors))
 
 
 def _load():

@@ -283,7 +283,7 @@ def ln_modulate(x: torch.Tensor, shift: torch.Tensor, scale: torch.Tensor, eps: 
     """``F.layer_norm(x, (C,), eps=eps) * (1 + scale) + shift`` for x (B, L, C) and shift / scale (B, C) or
     (B, 1, C); dual tensors in give a dual tensor out.  The result has ``out_dtype`` (default: the autocast
     dtype when autocast is on, else x's dtype)."""
-    if not torch.compiler.is_compiling():
+    if _native.takes(x, shift, scale):
         out = _native.ln_modulate(x, shift, scale, eps, out_dtype)
         if out is not None:
             return out
@@ -303,7 +303,7 @@ def ln_modulate(x: torch.Tensor, shift: torch.Tensor, scale: torch.Tensor, eps: 
 def gate_residual(x: torch.Tensor, gate: torch.Tensor, h: torch.Tensor) -> torch.Tensor:
     """``x + gate * h`` for x, h (B, L, C) and gate (B, C) or (B, 1, C); the result has x's dtype; dual tensors
     in give a dual tensor out."""
-    if not torch.compiler.is_compiling():
+    if _native.takes(x, gate, h):
         out = _native.gate_residual(x, gate, h)
         if out is not None:
             return out
@@ -320,7 +320,7 @@ def gelu(x: torch.Tensor) -> torch.Tensor:
     """GELU in its tanh form (the block's MLP), as one kernel for 16-bit CUDA tensors; a dual tensor in gives a dual tensor
     out.  Everything else (other types and devices, transforms the native path does not take) is
     ``torch.nn.functional.gelu``: the same function, with the same values, gradients and second derivatives."""
-    if not torch.compiler.is_compiling():
+    if _native.takes(x):
         out = _native.gelu(x)
         if out is not None:
             return out

@@ -12,6 +12,8 @@
 //   * anything else (tensor subclasses, dispatch modes, jit tracing, vmap / grad / nested transforms, arguments that the op
 //     rejects, CPU tensors) returns None, and the Python caller takes the general route, which also raises the exact errors.
 //
+// What Python sees first (torch.compile, __torch_function__) is sorted out in _native.takes.
+//
 // Semantics are those of the autograd.Functions in flash_attn_jvp.py, rms_norm.py and adaln.py: tangents are plain
 // inputs, backward differentiates the primal outputs only and once, tangent outputs carry no gradient (GELU, which stands in
 // for a library function, excepted).

@@ -80,7 +80,7 @@ def _is_dual_mode(*tensors):
 
 
 def flash_attn_func(q, k, v, softmax_scale=None):
-    if not torch.compiler.is_compiling():
+    if _native.takes(q, k, v):
         out = _native.attn_func(q, k, v, softmax_scale)
         if out is not None:
             return out
@@ -135,7 +135,7 @@ class FlashAttnQKVPackedFunc(torch.autograd.Function):
 def flash_attn_qkvpacked_func(qkv, softmax_scale=None):
     if qkv.dim() != 5 or qkv.shape[2] != 3:
         raise ValueError("expected a (B, L, 3, H, D) tensor")
-    if not torch.compiler.is_compiling():
+    if _native.takes(qkv):
         out = _native.attn_qkvpacked(qkv, softmax_scale)
         if out is not None:
             return out

@@ -59,7 +59,7 @@ class RmsNormFunc(torch.autograd.Function):
 
 def rms_norm(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-6) -> torch.Tensor:
     """RMSNorm over the last dim of a (B, L, H, D) tensor; a dual tensor in gives a dual tensor out."""
-    if not torch.compiler.is_compiling():
+    if _native.takes(x, weight):
         out = _native.rms_norm(x, weight, eps)
         if out is not None:
             return out

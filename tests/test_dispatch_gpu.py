@@ -5,7 +5,7 @@ import pytest
 import torch
 from torch.overrides import TorchFunctionMode
 
-from dmf_b200 import adaln, flash_attn_func, flash_attn_qkvpacked_func
+from dmf_b200 import _native, adaln, flash_attn_func, flash_attn_qkvpacked_func
 from dmf_b200.rms_norm import rms_norm
 
 pytestmark = pytest.mark.gpu
@@ -150,3 +150,29 @@ def test_saved_tensors_in_another_layout(op):
         out = fn(*args)
     with pytest.raises((RuntimeError, ValueError)):
         torch.autograd.grad(out, args, dout)
+
+
+class Named(torch.Tensor):
+    """A subclass without a Python dispatch key: only __torch_function__ sees its calls."""
+
+
+@pytest.mark.parametrize("op", ("attn", "packed", "rms", "gelu"))
+def test_subclasses_and_function_modes_see_the_op(op):
+    fn, args = _case(op)
+    want = fn(*args)
+    got = fn(args[0].as_subclass(Named), *args[1:])
+    assert type(got) is Named and torch.equal(got.as_subclass(torch.Tensor), want)
+    seen = []
+
+    class Spy(TorchFunctionMode):
+        def __torch_function__(self, func, types, a=(), kw=None):
+            seen.append(str(func))
+            return func(*a, **(kw or {}))
+
+    with Spy():
+        got = fn(*args)
+    assert torch.equal(got, want)
+    assert any(("gelu" if op == "gelu" else "dmf_b200") in s for s in seen), seen
+    with torch.device(DEV):                         # a function mode as well, but not one that looks at ops
+        assert _native.takes(*args) and not _native.takes(args[0].as_subclass(Named), *args[1:])
+        assert _native.takes(torch.nn.Parameter(args[0]))
