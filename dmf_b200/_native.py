@@ -4,6 +4,9 @@ one ``torch.func.jvp``.  Its functions return None for everything else, and the 
 ``takes`` comes before them: what torch.compile traces, and tensors or modes with a __torch_function__ of their own, have to see
 the ops of the general route.
 
+The module is built (if stale) and loaded by the first call with a CUDA tensor, like libdmf_attn.so: a program that runs none
+of the kernels needs neither the libraries nor a CUDA toolkit.
+
 With DMF_ATTN_CHECK=1 (which reads the device status word back after every call) every function returns None.
 """
 
@@ -11,6 +14,7 @@ from __future__ import annotations
 
 import importlib.util
 import os
+import threading
 
 import torch
 from torch.overrides import _get_current_function_mode_stack, has_torch_function
@@ -18,6 +22,9 @@ from torch.utils._device import DeviceContext
 
 from . import _lib
 from . import build as _build
+
+# DMF_ATTN_CHECK=1 reads the status word back after every call (synchronises; for tests and debugging).
+CHECK_EVERY_CALL = os.environ.get("DMF_ATTN_CHECK", "0") == "1"
 
 
 def takes(*tensors) -> bool:
@@ -28,26 +35,52 @@ def takes(*tensors) -> bool:
         return True
     # `with torch.device(...)` and set_default_device are function modes too, but concern factory functions only
     return (all(type(m) is DeviceContext for m in _get_current_function_mode_stack())
-            and all(type(t) is torch.Tensor or type(t).__torch_function__ is torch._C._disabled_torch_function_impl
+            and all(type(t) is torch.Tensor
+                    or getattr(type(t), "__torch_function__", None) is torch._C._disabled_torch_function_impl
                     for t in tensors))
 
 
-def _load():
-    _lib.load()                    # libdmf_attn.so first: built if stale, ABI version checked
-    spec = importlib.util.spec_from_file_location("_dmf_torch", _build.build_host())
-    module = importlib.util.module_from_spec(spec)
-    spec.loader.exec_module(module)
-    return module
+_module = None
+_lock = threading.Lock()
 
 
-_module = _load()
-launch_count, set_launch_count, set_status_word = _module.launch_count, _module.set_launch_count, _module.set_status_word
+def _loaded():
+    """The native module, built and loaded on first use."""
+    global _module
+    if _module is None:
+        with _lock:
+            if _module is None:
+                _lib.load()            # libdmf_attn.so first: built if stale, ABI version checked
+                spec = importlib.util.spec_from_file_location("_dmf_torch", _build.build_host())
+                module = importlib.util.module_from_spec(spec)
+                spec.loader.exec_module(module)
+                for name, stub in _stubs.items():      # later calls go straight to the native function
+                    if globals()[name] is stub and not CHECK_EVERY_CALL:
+                        globals()[name] = getattr(module, name)
+                _module = module
+    return _module
 
-# DMF_ATTN_CHECK=1 reads the status word back after every call (synchronises; for tests and debugging).
-CHECK_EVERY_CALL = os.environ.get("DMF_ATTN_CHECK", "0") == "1"
 
-if CHECK_EVERY_CALL:
-    attn_func = attn_qkvpacked = rms_norm = ln_modulate = gate_residual = gelu = lambda *args: None
-else:
-    attn_func, attn_qkvpacked = _module.attn_func, _module.attn_qkvpacked
-    rms_norm, ln_modulate, gate_residual, gelu = _module.rms_norm, _module.ln_modulate, _module.gate_residual, _module.gelu
+def _stub(name):
+    def first_call(*args):
+        if CHECK_EVERY_CALL or not any(isinstance(a, torch.Tensor) and a.is_cuda for a in args):
+            return None
+        return getattr(_loaded(), name)(*args)
+    return first_call
+
+
+_stubs = {name: _stub(name) for name in ("attn_func", "attn_qkvpacked", "rms_norm", "ln_modulate", "gate_residual", "gelu")}
+globals().update(_stubs)
+
+
+def set_status_word(index: int, pointer: int) -> None:
+    _loaded().set_status_word(index, pointer)
+
+
+def launch_count() -> int:
+    return 0 if _module is None else _module.launch_count()
+
+
+def set_launch_count(n: int) -> None:
+    if n or _module is not None:
+        _loaded().set_launch_count(n)
