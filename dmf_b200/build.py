@@ -1,8 +1,9 @@
 """Build the C-ABI shared library (dmf_b200/libdmf_attn.so) with nvcc for sm_100a, and the native host path of the Python
-surface (dmf_b200/_dmf_torch.so, csrc/torch_host.cpp) with the C++ compiler.
+surface (dmf_b200/_dmf_torch.*.so, csrc/torch_host.cpp) with the C++ compiler.
 
 Both are built in-tree so that they travel with the source snapshot.  The library has no Python or torch dependency; the
-host module links it and torch.  ``python -m dmf_b200.build`` builds them by hand.
+host module links it and torch, and has the Python and torch it was built for in its name: under others it is built anew.
+``python -m dmf_b200.build`` builds them by hand.
 """
 
 from __future__ import annotations
@@ -19,7 +20,6 @@ CSRC = PKG / "csrc"
 INCLUDE = PKG.parent / "include"
 LIB = PKG / "libdmf_attn.so"
 
-HOST_MODULE = PKG / "_dmf_torch.so"
 HOST_SOURCE = CSRC / "torch_host.cpp"
 
 SOURCES = ["dmf_attn.cu", "attn_fwd_duo.cu", "dmf_adaln.cu", "dmf_step.cu"]
@@ -37,6 +37,15 @@ def find_nvcc() -> str | None:
     return cand if cand and Path(cand).exists() else None
 
 
+def host_module() -> Path:
+    """The host module's path: it is compiled against torch's C++ internals and CPython's, so their versions name it."""
+    import sysconfig
+
+    import torch
+    torch_id = f"torch{torch.__version__}-{(torch.version.git_version or '')[:8]}-cxx{int(torch.compiled_with_cxx11_abi())}"
+    return PKG / f"_dmf_torch.{sysconfig.get_config_var('SOABI')}.{torch_id}.so"
+
+
 def _older(target: Path, deps) -> bool:
     return not target.exists() or any(d.stat().st_mtime > target.stat().st_mtime for d in deps)
 
@@ -46,7 +55,7 @@ def _stale() -> bool:
 
 
 def _host_stale() -> bool:
-    return _older(HOST_MODULE, [HOST_SOURCE, *(CSRC / "compat").rglob("*.hpp"), *INCLUDE.glob("*.h")])
+    return _older(host_module(), [HOST_SOURCE, *(CSRC / "compat").rglob("*.hpp"), *INCLUDE.glob("*.h")])
 
 
 def build(force: bool = False, verbose: bool = False) -> Path:
@@ -86,22 +95,22 @@ def build(force: bool = False, verbose: bool = False) -> Path:
 
 def build_host(force: bool = False) -> Path:
     """Compile the native host path (torch_host.cpp) if it is missing or older than its sources; same locking as build()."""
-    lib = build()
+    lib, target = build(), host_module()
     if not force and not _host_stale():
-        return HOST_MODULE
+        return target
     import sysconfig
 
     import torch
     root = Path(torch.__file__).resolve().parent
     nvcc = find_nvcc()
     if nvcc is None:
-        raise RuntimeError("no CUDA toolkit: cannot build dmf_b200/_dmf_torch.so")
+        raise RuntimeError(f"no CUDA toolkit: cannot build {target.name}")
     with open(PKG / ".build.lock", "w") as lock:
         fcntl.flock(lock, fcntl.LOCK_EX)
         try:
             if not force and not _host_stale():
-                return HOST_MODULE
-            tmp = HOST_MODULE.with_name(f".{HOST_MODULE.name}.{os.getpid()}.tmp")
+                return target
+            tmp = target.with_name(f".{target.name}.{os.getpid()}.tmp")
             includes = [root / "include", root / "include" / "torch" / "csrc" / "api" / "include",
                         sysconfig.get_paths()["include"], Path(nvcc).resolve().parent.parent / "include", CSRC / "compat"]
             cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
@@ -113,10 +122,10 @@ def build_host(force: bool = False) -> Path:
             if res.returncode != 0:
                 tmp.unlink(missing_ok=True)
                 raise RuntimeError(f"{cmd[0]} failed ({res.returncode}):\n{res.stdout}\n{res.stderr}")
-            os.replace(tmp, HOST_MODULE)
+            os.replace(tmp, target)
         finally:
             fcntl.flock(lock, fcntl.LOCK_UN)
-    return HOST_MODULE
+    return target
 
 
 if __name__ == "__main__":

@@ -1,4 +1,5 @@
-"""What a program gets without the CUDA toolkit and without built libraries: everything that runs no kernel."""
+"""What a program gets without the CUDA toolkit and without built libraries - everything that runs no kernel - and which
+build of the host module it loads."""
 
 import os
 import shutil
@@ -43,3 +44,22 @@ print("ran")
 """.format(root=str(bare_tree)))
     assert res.returncode == 0 and "ran" in res.stdout, res.stderr[-2000:]
     assert not list(bare_tree.rglob("*.so"))
+
+
+@pytest.mark.parametrize("change", ["torch version", "torch build", "C++ ABI", "Python"])
+def test_a_host_module_built_for_another_torch_or_python_is_not_loaded(monkeypatch, change):
+    import sysconfig
+
+    import torch
+
+    from dmf_b200 import build
+    here = build.host_module()
+    if change == "torch version":
+        monkeypatch.setattr(torch, "__version__", "2.99.0+cu131")
+    elif change == "torch build":
+        monkeypatch.setattr(torch.version, "git_version", "0" * 40)
+    elif change == "C++ ABI":
+        monkeypatch.setattr(torch, "compiled_with_cxx11_abi", lambda now=torch.compiled_with_cxx11_abi(): not now)
+    else:
+        monkeypatch.setattr(sysconfig, "get_config_var", lambda name: "cpython-399-x86_64-linux-gnu")
+    assert build.host_module() != here and build._host_stale()
