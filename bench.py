@@ -76,10 +76,10 @@ def _peaks():
     return {"tflops": 1590.0, "tflops_sustained": 1400.0, "hbm_gbs": 6650.0, "source": "fallback"}
 
 
-def _kernel_name(op, D, L):
+def _kernel_name(op, D, L, B=None, H=None):
     """The kernel instance the library's launcher picks for this shape, asked of the library itself."""
     from dmf_b200 import _lib
-    return _lib.kernel_name(op, L, L, D)
+    return _lib.kernel_name(op, L, L, D, batch=B, heads=H)
 
 
 def _traffic(workload):
@@ -325,7 +325,7 @@ def _secondary(dev, peaks, steps):
             ms = _time_launches(fn, steps)
             r = _attn_roofline(op, B, L, H, D, ms, peaks)
             out[f"{wl}_{op}"] = {"ms": ms, "tflops": r["tflops"], "gbs": r["gbs"], "bound": r["bound"], "frac": r["frac"],
-                                 "kernel": _kernel_name(op, D, L)}
+                                 "kernel": _kernel_name(op, D, L, B, H)}
         if wl == "C3":
             # q / k RMS norm with tangents on the packed projection, and the adaLN ops of one block with tangents
             qkv = torch.randn(B, L, 3, H, D, device=dev, generator=gen).to(torch.bfloat16)
@@ -584,7 +584,7 @@ def run_ours(args):
         "frac_of_nominal_2250": roof["tflops"] / 2250.0,
         "algorithmic_flops_per_launch": fl, "algorithmic_bytes_per_launch": roof["bytes"],
         "hbm_gbs_achieved": roof["gbs"], "frac_of_hbm": roof["gbs"] / peaks["hbm_gbs"],
-        "kernel": _kernel_name(op, D, L),
+        "kernel": _kernel_name(op, D, L, B, H),
         "sustained": sustained,
     }
     del ins, q, k, v, tq, tk, tv, out

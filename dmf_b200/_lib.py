@@ -27,6 +27,7 @@ EXPORTS = (
     "dmf_attn_bwd", "dmf_attn_bwd_static", "dmf_attn_bwd_workspace_bytes", "dmf_attn_check_status_word",
     "dmf_attn_validate_fwd", "dmf_attn_validate_bwd",
     "dmf_attn_fwd_dual_f32out", "dmf_attn_selftest_wait_limit", "dmf_attn_kernel_name",
+    "dmf_attn_kernel_name_for",
     "dmf_rmsnorm_fwd", "dmf_rmsnorm_bwd", "dmf_rmsnorm_bwd_workspace_bytes",
     "dmf_ln_modulate_fwd", "dmf_ln_modulate_bwd", "dmf_adaln_bwd_workspace_bytes",
     "dmf_gate_residual_fwd", "dmf_gate_residual_bwd", "dmf_gelu",
@@ -177,6 +178,8 @@ def load() -> C.CDLL:
         lib.dmf_attn_status_string.argtypes = [C.c_int]
         lib.dmf_attn_selftest_wait_limit.restype = C.c_int
         lib.dmf_attn_selftest_wait_limit.argtypes = [C.c_int64, C.c_void_p, C.c_void_p, C.c_void_p]
+        lib.dmf_attn_kernel_name_for.restype = C.c_int
+        lib.dmf_attn_kernel_name_for.argtypes = [C.c_int32] * 7 + [C.c_char_p, C.c_size_t]
         lib.dmf_attn_kernel_name.restype = C.c_int
         lib.dmf_attn_kernel_name.argtypes = [C.c_int32] * 5 + [C.c_char_p, C.c_size_t]
         for name in ("dmf_attn_fwd_dual", "dmf_attn_fwd", "dmf_attn_fwd_dual_f32out"):
@@ -218,11 +221,16 @@ def load() -> C.CDLL:
         return lib
 
 
-def kernel_name(op: str, seqlen_q: int, seqlen_kv: int, head_dim: int, dtype: int = BF16) -> str:
-    """The kernel template instance the launcher picks for this problem (op: 'dual', 'fwd' or 'bwd')."""
+def kernel_name(op: str, seqlen_q: int, seqlen_kv: int, head_dim: int, dtype: int = BF16, batch: int | None = None,
+                heads: int | None = None) -> str:
+    """The kernel template instance the launcher picks for this problem (op: 'dual', 'fwd' or 'bwd'); without batch and
+    heads, which the plain forward's choice can depend on, for as many heads as fill the GPU once."""
     buf = C.create_string_buffer(256)
-    check(load().dmf_attn_kernel_name({"dual": 0, "fwd": 1, "bwd": 2}[op], seqlen_q, seqlen_kv, head_dim, dtype,
-                                      buf, len(buf)))
+    code, shape = {"dual": 0, "fwd": 1, "bwd": 2}[op], (seqlen_q, seqlen_kv, head_dim, dtype, buf, len(buf))
+    if batch is None or heads is None:
+        check(load().dmf_attn_kernel_name(code, *shape))
+    else:
+        check(load().dmf_attn_kernel_name_for(code, batch, heads, *shape))
     return buf.value.decode()
 
 

@@ -262,7 +262,7 @@ bool pair_kernel_enabled() {
   return enabled;
 }
 
-// Which kernel template the launcher picks for a problem; one rule for the launch and for dmf_attn_kernel_name.
+// Which kernel template the launcher picks for a problem; one rule for the launch and for dmf_attn_kernel_name_for.
 bool fwd_uses_pair(bool dual, int tail, int seqlen_q) {
   return dual && tail >= 0 && tail <= 32 && ((seqlen_q / kBlockQ) % 2 == 0) && pair_kernel_enabled();
 }
@@ -838,8 +838,11 @@ int run_selftest_wait_limit(int64_t limit_cycles, int32_t* status_word, int32_t*
 
 // ---- name of the kernel a call would launch ----
 
-int kernel_name(int op, int seqlen_q, int seqlen_kv, int head_dim, int dtype, char* buf, size_t len) {
+// batch_heads < 1: as many heads as fill the GPU once with two query tiles per CTA
+int kernel_name(int op, int64_t batch_heads, int seqlen_q, int seqlen_kv, int head_dim, int dtype, char* buf, size_t len) {
   if (buf == nullptr || len == 0) return DMF_ATTN_ERR_NULL;
+  int sm_count = 0;
+  if (device_info(&sm_count) != DMF_ATTN_OK) sm_count = 148;
   if (dtype != DMF_ATTN_BF16 && dtype != DMF_ATTN_FP16) return DMF_ATTN_ERR_DTYPE;
   const int tail = tail_of(head_dim);
   if (tail < 0) return DMF_ATTN_ERR_HEAD_DIM;
@@ -848,7 +851,8 @@ int kernel_name(int op, int seqlen_q, int seqlen_kv, int head_dim, int dtype, ch
   if (op == 0 || op == 1) {
     const char* kind = op == 0 ? "dual" : "plain";
     const int q_tiles = seqlen_q / kBlockQ, units = (q_tiles + 1) / 2;
-    if (fwd_uses_duo(op == 0, head_dim, units < 148 ? 148 / units : 1, q_tiles, 148)) {  // as many heads as fill the GPU once
+    if (batch_heads < 1) batch_heads = units < sm_count ? sm_count / units : 1;
+    if (fwd_uses_duo(op == 0, head_dim, batch_heads, q_tiles, sm_count)) {
       std::snprintf(buf, len, "attn_fwd_duo_kernel<%s, TAIL=%d> (two query tiles per CTA)", t, tail);
     } else if (fwd_uses_pair(op == 0, tail, seqlen_q)) {
       const bool is_short = tail == 16 && seqlen_kv <= kShortMaxBlocks * kBlockKV;
@@ -1048,9 +1052,14 @@ DMF_API int dmf_trace_read_bwd_fused(unsigned long long* out, size_t count) {
 }
 #endif
 
+DMF_API int dmf_attn_kernel_name_for(int32_t op, int32_t batch, int32_t heads, int32_t seqlen_q, int32_t seqlen_kv,
+                                     int32_t head_dim, int32_t dtype, char* buf, size_t len) {
+  if (batch < 1 || heads < 1) return DMF_ATTN_ERR_SHAPE;
+  return kernel_name(op, static_cast<int64_t>(batch) * heads, seqlen_q, seqlen_kv, head_dim, dtype, buf, len);
+}
 DMF_API int dmf_attn_kernel_name(int32_t op, int32_t seqlen_q, int32_t seqlen_kv, int32_t head_dim, int32_t dtype,
                                  char* buf, size_t len) {
-  return kernel_name(op, seqlen_q, seqlen_kv, head_dim, dtype, buf, len);
+  return kernel_name(op, 0, seqlen_q, seqlen_kv, head_dim, dtype, buf, len);
 }
 
 DMF_API int dmf_attn_validate_fwd(const dmf_attn_fwd_args* args, int dual) { return validate_fwd(args, dual != 0); }

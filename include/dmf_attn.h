@@ -213,11 +213,16 @@ int dmf_attn_check_status_word(const int32_t* status_word, void* stream, int32_t
  * (expect 0), a second thread's longer wait succeeded (expect 0: it sees the abort flag), a wait
  * on a signalled barrier succeeded (expect 1), cycles the first thread waited}.
  *
- * dmf_attn_kernel_name: the kernel template instance the launcher picks for a problem, as text
- * (op: 0 = fused forward + tangent, 1 = plain forward, 2 = backward).
+ * dmf_attn_kernel_name_for: the kernel template instance the launcher picks for a problem on the
+ * current device (on a B200 where there is none), as text (op: 0 = fused forward + tangent, 1 =
+ * plain forward, 2 = backward).  dmf_attn_kernel_name: the same without batch and heads, which the
+ * plain forward's choice depends on at odd tile counts and head_dim above 96: for as many heads as
+ * fill the GPU once.
  */
 int dmf_attn_fwd_dual_f32out(const dmf_attn_fwd_args* args);
 int dmf_attn_selftest_wait_limit(int64_t limit_cycles, int32_t* status_word, int32_t* result, void* stream);
+int dmf_attn_kernel_name_for(int32_t op, int32_t batch, int32_t heads, int32_t seqlen_q, int32_t seqlen_kv,
+                             int32_t head_dim, int32_t dtype, char* buf, size_t len);
 int dmf_attn_kernel_name(int32_t op, int32_t seqlen_q, int32_t seqlen_kv, int32_t head_dim, int32_t dtype,
                          char* buf, size_t len);
 
