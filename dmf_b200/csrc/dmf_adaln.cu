@@ -5,6 +5,7 @@
 #include <type_traits>
 
 #include "adaln.cuh"
+#include "attn_launch.h"
 #include "dmf_adaln.h"
 #include "dmf_attn.h"
 #include "gelu.cuh"
@@ -191,13 +192,8 @@ int run_ln_modulate_bwd(const dmf_ln_modulate_bwd_args* a) {
     return with_width(a->channels, [&](auto nv) {
       constexpr int NV = decltype(nv)::value;
       constexpr int kSmem = (1 + 2 * kAdaWarps) * NV * 128 * static_cast<int>(sizeof(float));
-      static bool configured = false;  // per instantiation
-      if (!configured) {
-        if (cudaFuncSetAttribute(ln_modulate_bwd_kernel<TW, TN, NV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 kSmem) != cudaSuccess)
-          return static_cast<int>(DMF_ATTN_ERR_LAUNCH);
-        configured = true;
-      }
+      static bool done[64];  // per instantiation
+      if (!allow_smem(ln_modulate_bwd_kernel<TW, TN, NV>, kSmem, done)) return static_cast<int>(DMF_ATTN_ERR_LAUNCH);
       ln_modulate_bwd_kernel<TW, TN, NV><<<grid, kAdaThreads, kSmem, stream>>>(p);
       return launched();
     });

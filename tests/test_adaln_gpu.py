@@ -204,3 +204,17 @@ def test_gate_residual_forward_widths_and_row_counts(wide, narrow, B, L, Cn):
             # one rounding of the result (half a unit in the last place), and two of the fp32 sums of its terms
             bound = 1.01 * half * sum(terms).abs() + 3 * 2.0 ** -24 * sum(t.abs() for t in terms)
             assert bool(((got.double() - sum(terms)).abs() <= bound).all())
+
+
+@pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs a second GPU")
+def test_ln_modulate_backward_on_every_gpu_of_a_process():
+    """Its kernel needs 78 KB of shared memory at the largest width, which is granted device by device."""
+    grads = []
+    for i in range(torch.cuda.device_count()):
+        g = torch.Generator().manual_seed(5)
+        x, shift, scale = (torch.randn(*s, generator=g).to(f"cuda:{i}").requires_grad_(True)
+                           for s in ((2, 64, 1152), (2, 1152), (2, 1152)))
+        y = adaln.ln_modulate(x, shift, scale, out_dtype=BF16)
+        grads.append([t.cpu() for t in torch.autograd.grad(y.float().square().sum(), (x, shift, scale))])
+    for other in grads[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(other, grads[0], strict=True))
