@@ -15,7 +15,7 @@ namespace {
 using namespace dmf;
 
 int sm_count_of_current_device(int* sm_count) {
-  static int cached_dev = -1, cached_sms = 0, cached_ok = 0;  // one device per process in practice
+  static thread_local int cached_dev = -1, cached_sms = 0, cached_ok = 0;  // a thread rarely changes its device
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return DMF_ATTN_ERR_DEVICE;
   if (dev != cached_dev) {
@@ -215,10 +215,10 @@ bool gate_vec8(const dmf_gate_residual_args* a, bool dual, bool tmod) {
 }
 
 // 16 rows per block (8 to 32 time the same), fewer where that leaves SMs without a few blocks, down to one row per thread
-int gate_rows_per_block(int batch, int seqlen, int lanes) {
-  constexpr int64_t kWantBlocks = 4 * 148;
+int gate_rows_per_block(int batch, int seqlen, int lanes, int sms) {
+  const int64_t want_blocks = 4 * static_cast<int64_t>(sms);
   int rpb = 16;
-  while (rpb > lanes && static_cast<int64_t>(batch) * ((seqlen + rpb - 1) / rpb) < kWantBlocks) rpb /= 2;
+  while (rpb > lanes && static_cast<int64_t>(batch) * ((seqlen + rpb - 1) / rpb) < want_blocks) rpb /= 2;
   return rpb > lanes ? rpb : lanes;
 }
 
@@ -255,7 +255,7 @@ int run_gate_residual_fwd(const dmf_gate_residual_args* a) {
   cudaStream_t stream = static_cast<cudaStream_t>(a->stream);
   if (gate_vec8(a, dual, tmod)) {
     const int nvec = a->channels / 8, threads = gate_row_threads(nvec) * gate_row_lanes(nvec);
-    p.rows_per_block = gate_rows_per_block(a->batch, a->seqlen, gate_row_lanes(nvec));
+    p.rows_per_block = gate_rows_per_block(a->batch, a->seqlen, gate_row_lanes(nvec), sms);
     const dim3 grid((a->seqlen + p.rows_per_block - 1) / p.rows_per_block, a->batch);
     return with_types(a->wide_dtype, a->narrow_dtype, [&](auto tw, auto tn) {
       using TW = decltype(tw);
