@@ -81,6 +81,11 @@ def launch_count() -> int:
     return 0 if _module is None else _module.launch_count()
 
 
+def add_launches(n: int) -> None:
+    """One step, unlike reading, adding and setting: the native functions count without the GIL, backward on other threads."""
+    _loaded().add_launches(n)
+
+
 def set_launch_count(n: int) -> None:
     if n or _module is not None:
         _loaded().set_launch_count(n)

@@ -116,7 +116,7 @@ def ln_modulate_fwd_raw(x, tx, shift, scale, tshift, tscale, eps: float, out_dty
         a.shift, a.scale = _mod(shift), _mod(scale)
         a.tshift, a.tscale = (_mod(tshift), _mod(tscale)) if tx is not None else (_mod(None), _mod(None))
         _lib.check(_lib.load().dmf_ln_modulate_fwd(C.byref(a)))
-        _ops.launch_count += 1
+        _ops._count(1)
     return y, ty
 
 
@@ -137,7 +137,7 @@ def ln_modulate_bwd_raw(dy, x, scale, eps: float):
         a.dshift, a.dscale = dmod[0].data_ptr(), dmod[1].data_ptr()
         a.workspace, a.workspace_bytes = ws.data_ptr(), nbytes
         _lib.check(_lib.load().dmf_ln_modulate_bwd(C.byref(a)))
-        _ops.launch_count += 2
+        _ops._count(2)
     return dx, dmod[0], dmod[1]
 
 
@@ -162,7 +162,7 @@ def gate_residual_fwd_raw(x, tx, h, th, gate, tgate):
         a.x, a.h, a.out, a.gate = _rows(x), _rows(h), _rows(out), _mod(gate)
         a.tx, a.th, a.tout, a.tgate = _rows(tx if dual else None), _rows(th if dual else None), _rows(tout), _mod(tgate if dual else None)
         _lib.check(_lib.load().dmf_gate_residual_fwd(C.byref(a)))
-        _ops.launch_count += 1
+        _ops._count(1)
     return out, tout
 
 
@@ -182,7 +182,7 @@ def gate_residual_bwd_raw(dout, h, gate):
         a.dgate = dgate.data_ptr()
         a.workspace, a.workspace_bytes = ws.data_ptr(), nbytes
         _lib.check(_lib.load().dmf_gate_residual_bwd(C.byref(a)))
-        _ops.launch_count += 2
+        _ops._count(2)
     return dh, dgate
 
 

@@ -996,5 +996,6 @@ PYBIND11_MODULE(_dmf_torch, m) {
     g_status_word[device].store(reinterpret_cast<int32_t*>(ptr), std::memory_order_release);
   });
   m.def("launch_count", [] { return g_launches.load(std::memory_order_relaxed); });
+  m.def("add_launches", [](int64_t n) { g_launches.fetch_add(n, std::memory_order_relaxed); });
   m.def("set_launch_count", [](int64_t n) { g_launches.store(n, std::memory_order_relaxed); });
 }

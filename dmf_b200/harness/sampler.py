@@ -65,6 +65,6 @@ class GraphedSampler:
         self.z.copy_(z, non_blocking=True)
         self.y.copy_(y, non_blocking=True)
         self.graph.replay()
-        _ops.launch_count += self.launches
+        _ops._count(self.launches)
         _ops.poll_device_status(self.z.device)
         return self.out

@@ -28,7 +28,7 @@ _DTYPES = {torch.bfloat16: _lib.BF16, torch.float16: _lib.FP16}
 
 class _Module(types.ModuleType):
     """``ops.launch_count``: kernel launches of this package since import (a backward call counts two).  The counter lives
-    in the native host path, which makes most of them."""
+    in the native host path, which makes most of them; set it to reset it, add to it with ``_count``."""
 
     @property
     def launch_count(self) -> int:
@@ -43,7 +43,7 @@ sys.modules[__name__].__class__ = _Module
 
 
 def _count(n: int) -> None:
-    _native.set_launch_count(_native.launch_count() + n)
+    _native.add_launches(n)
 
 
 # One int32 per device that kernels write to when a device-side wait runs out.

@@ -48,4 +48,4 @@ class FlatAdamW:
         with torch.cuda.device(flat_param.device):
             a.stream = torch.cuda.current_stream(flat_param.device).cuda_stream
             _lib.check(_lib.load().dmf_step_tail(C.byref(a)))
-        _ops.launch_count += 1
+        _ops._count(1)

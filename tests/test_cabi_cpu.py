@@ -176,3 +176,22 @@ def test_python_surface_has_no_cpu_path():
         adaln.ln_modulate(x, mod, mod)
     with pytest.raises(RuntimeError):
         adaln.gate_residual(x, mod, x)
+
+
+def test_launches_counted_by_several_threads_add_up():
+    import sys
+    import threading
+
+    from dmf_b200 import ops
+    before, interval = ops.launch_count, sys.getswitchinterval()
+    sys.setswitchinterval(1e-6)
+    try:
+        threads = [threading.Thread(target=lambda: [ops._count(1) for _ in range(20000)]) for _ in range(4)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        assert ops.launch_count - before == 80000
+    finally:
+        sys.setswitchinterval(interval)
+        ops.launch_count = before
