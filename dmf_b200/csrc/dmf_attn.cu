@@ -153,8 +153,18 @@ int make_map(CUtensorMap* map, const dmf_attn_tensor& t, int dtype, int batch, i
   cuuint32_t elem_strides[4] = {1, 1, 1, 1};
   const CUtensorMapDataType dt =
       dtype == DMF_ATTN_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
-  const CUresult r = encode(map, dt, 4, t.ptr, dims, strides, box, elem_strides, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                            swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  auto run = [&] {
+    return encode(map, dt, 4, t.ptr, dims, strides, box, elem_strides, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  };
+  CUresult r = run();
+  if (r != CUDA_SUCCESS) {
+    // a driver call: it needs the device's context current to this thread, and on a thread without a runtime call so far
+    // (an autograd worker whose memory all comes from a cache) nothing has bound it yet; cudaSetDevice does
+    int dev = -1;
+    if (cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess) r = run();
+    (void)cudaGetLastError();
+  }
   return r == CUDA_SUCCESS ? DMF_ATTN_OK : DMF_ATTN_ERR_TENSOR_MAP;
 }
 

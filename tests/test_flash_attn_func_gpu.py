@@ -166,3 +166,28 @@ def test_long_sequence_backward_replays_in_a_cuda_graph():
         torch.cuda.synchronize()
         assert torch.equal(sk.grad, eager[1]) and torch.equal(sv.grad, eager[2])
         assert orc.rel_l2(sq.grad.float().cpu(), eager[0].float().cpu()) < 1e-3
+
+
+def test_first_cuda_work_of_a_thread():
+    """A thread that has made no CUDA call yet (an autograd worker, a server's) has no driver context until one is bound; its
+    memory may all come from the caching allocator."""
+    import threading
+    qkv = torch.randn(2, 256, 3, 2, 64, device="cuda:0", dtype=torch.bfloat16)
+    q, k, v = (x.contiguous() for x in qkv.unbind(2))
+    want = flash_attn_func(q, k, v)
+    flash_attn_func(q, k, v)                                         # its blocks are in the cache now
+    torch.cuda.synchronize()
+    got, errors = [], []
+
+    def work():
+        try:
+            got.append(flash_attn_func(q, k, v))
+            torch.cuda.current_stream().synchronize()
+        except Exception as e:  # noqa: BLE001
+            errors.append(e)
+
+    for _ in range(3):
+        t = threading.Thread(target=work)
+        t.start()
+        t.join()
+    assert not errors and all(torch.equal(o, want) for o in got)
