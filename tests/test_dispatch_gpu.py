@@ -3,6 +3,7 @@ gradients, tangents that are differentiated, saved-tensor hooks, tensor subclass
 
 import pytest
 import torch
+import torch.utils.checkpoint
 from torch.overrides import TorchFunctionMode
 
 from dmf_b200 import _native, adaln, flash_attn_func, flash_attn_qkvpacked_func
@@ -176,3 +177,23 @@ def test_subclasses_and_function_modes_see_the_op(op):
     with torch.device(DEV):                         # a function mode as well, but not one that looks at ops
         assert _native.takes(*args) and not _native.takes(args[0].as_subclass(Named), *args[1:])
         assert _native.takes(torch.nn.Parameter(args[0]))
+
+
+@pytest.mark.parametrize("op", ALL)
+@pytest.mark.parametrize("reentrant", [True, False])
+def test_checkpointed_calls(op, reentrant):
+    """Recomputation in backward: without reentry it runs inside a saved-tensor hook, and needs autograd as usual there."""
+    fn, args = _case(op)
+    args = [a.requires_grad_(True) for a in args]
+    body = lambda *a: fn(a[0] * 2, *a[1:]).sin()
+
+    def gradients(out):
+        for a in args:
+            a.grad = None
+        out.backward(torch.ones_like(out))
+        return [a.grad for a in args]
+
+    plain = gradients(body(*args))
+    again = gradients(torch.utils.checkpoint.checkpoint(body, *args, use_reentrant=reentrant))
+    for a, b in zip(plain, again, strict=True):
+        assert torch.equal(a, b)
